@@ -155,7 +155,7 @@ int rec_initial(gs_plan* p, const double* h, const int* rcv, const double* wgt, 
     GS_TRY(rcopy(p, &r->wgt0, wgt, Rn));
     GS_TRY(rcopy(p, &r->dist0, dist, Rn));
     GS_TRY(rcopy(p, &r->rslot0, rslot, Rn));
-    GS_TRY(rcopy(p, &r->order0, order, n));
+    if (flow_needs_order(p)) GS_TRY(rcopy(p, &r->order0, order, n));
     GS_TRY(rcopy(p, &r->q0, q0, n));
     GS_TRY(rcopy(p, &r->sea, sea, n));
     r->order_ok = order_ok;
@@ -209,7 +209,7 @@ int rec_pass_solve(gs_plan* p, int t, const int* order, int order_ok, const doub
     GS_TRY(rcopy(p, &q->rcv, (const int*)p->rcv, Rn));
     GS_TRY(rcopy(p, &q->wgt, (const double*)p->wgt, Rn));
     GS_TRY(rcopy(p, &q->rslot, (const int8_t*)p->rslot, Rn));
-    GS_TRY(rcopy(p, &q->order, order, n));
+    if (flow_needs_order(p)) GS_TRY(rcopy(p, &q->order, order, n));
     GS_TRY(rcopy(p, &q->x, x, n));
     return GS_OK;
 }
@@ -488,7 +488,7 @@ int adjoint_step(gs_plan* p, int slot, double* lam, const double* rain, double k
             launch(p, k_cascade_gx, G, B, n, (const double*)r.hold, (const double*)q.wf, (const double*)gfal,
                    (const double*)gfa, dt, gx);
             GS_LAUNCH();
-            GS_TRY(sweep_flow_adjoint(p, q.rcv, q.wgt, q.order, gx, y));
+            GS_TRY(sweep_flow_adjoint(p, q.rcv, q.wgt, q.rslot, q.order, gx, y));
             launch(p, k_edge_gw, G, B, n, p->R, (const int*)q.rcv, (const double*)q.wgt, (const double*)q.x,
                    (const double*)y, 0, p->adj_er);
             GS_LAUNCH();
@@ -501,7 +501,7 @@ int adjoint_step(gs_plan* p, int slot, double* lam, const double* rain, double k
     }
     // initial solve: fal = q0 (+ cascade increments), FA_0 = q0 dt
     if (r.npass > 0) launch(p, k_axpy_acc, G, B, n, dt, (const double*)gfa, gfal);
-    GS_TRY(sweep_flow_adjoint(p, r.rcv0, r.wgt0, r.order0, gfal, y));
+    GS_TRY(sweep_flow_adjoint(p, r.rcv0, r.wgt0, r.rslot0, r.order0, gfal, y));
     if (gbl) launch(p, k_gbl, G, B, n, (const uint8_t*)r.sea, (const double*)y, gbl);
     launch(p, k_edge_gw, G, B, n, p->R, (const int*)r.rcv0, (const double*)r.wgt0, (const double*)r.q0,
            (const double*)y, 1, p->adj_gw);

@@ -274,6 +274,13 @@ static int read_flag(gs_plan* p, int* out) {
     return GS_OK;
 }
 
+// outcome of a flow sweep whose status came back with a synchronisation
+static int flow_status(gs_plan* p, int st) {
+    if (!flow_needs_order(p)) return tile_status_check(p, st, "flow sweep did not complete");
+    if (st != 0) set_error(st, "ordered flow sweep did not complete");
+    return st;
+}
+
 int flow_accumulation(gs_plan* p, const double* h, const double* bl, double sealevel, double ofill,
                       double dt, double* fal, double* fill_fal, double* water, double* lfill,
                       int* pit_ids, int* flat_dirs, int* rcv_i, double* dist_i, double* wgt_i,
@@ -291,8 +298,8 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
         StreamSwap sw(p, p->side_a, p->cub_tmp2);
         GS_TRY(flow_direction(p, h, false, nullptr, nullptr, nullptr, sealevel, rcv_i, dist_i, wgt_i,
                               p->rslot_i, nullptr, nullptr));
-        GS_TRY(flow_order(p, h, p->order_i));
-        GS_TRY(flow_prepare(p, rcv_i, wgt_i, p->rslot_i, fal, p->order_i, bad_a));
+        if (flow_needs_order(p)) GS_TRY(flow_order(p, h, p->order_i));
+        GS_TRY(flow_prepare(p, TG_SNAP, rcv_i, wgt_i, p->rslot_i, fal, h, nullptr, p->order_i, bad_a));
     }
     GS_CUDA(cudaEventRecord(p->ev_a, p->side_a));
     GS_TRY(fill_elevation(p, h, sealevel, ofill, lfill, pit_ids, flat_dirs, st, true, sea, false, bl));
@@ -310,7 +317,7 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
     int cyc = 0;
     // the sweep's status is read at the next synchronisation (the lakes flag)
     int* sweep_st = p->h_pinned + 10;
-    GS_TRY(flow_run(p, rcv_i, wgt_i, p->rslot_i, p->nfa, fal, &cyc, p->order_i, ok_i, sweep_st));
+    GS_TRY(flow_run(p, TG_SNAP, rcv_i, wgt_i, p->rslot_i, p->nfa, fal, &cyc, p->order_i, ok_i, sweep_st));
     GS_TRY(rec_initial(p, h, rcv_i, wgt_i, dist_i, p->rslot_i, p->order_i, ok_i, fal, sea));
     int total_cycles = cyc;
     launch(p, k_copy, G, B, (int64_t)n, h, p->wf);
@@ -326,10 +333,7 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
     std::vector<uint8_t> lakes(nm, 0);
     GS_CUDA(cudaMemcpyAsync(lakes.data(), p->mlakes, nm, cudaMemcpyDeviceToHost, p->stream));
     GS_CUDA(cudaStreamSynchronize(p->stream));
-    if (*sweep_st != 0) {
-        set_error(*sweep_st, "ordered flow sweep did not complete");
-        return *sweep_st;
-    }
+    GS_TRY(flow_status(p, *sweep_st));
     bool anyvol = false;
     for (int m = 0; m < nm; m++) anyvol = anyvol || lakes[m];
     int passes = 0, solves = 0;
@@ -345,6 +349,7 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
         double* FA = p->q;
         launch(p, k_scale, G, B, (int64_t)n, (const double*)fal, dt, FA);
         int step = 0;
+        bool solving = false;   // a sweep's status is still to be read
         auto any = [](const std::vector<uint8_t>& v) {
             for (uint8_t x : v)
                 if (x) return true;
@@ -364,6 +369,8 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
             GS_CUDA(cudaMemcpyAsync(p->h_mflags, p->mflags, sizeof(int) * nm, cudaMemcpyDeviceToHost, p->stream));
             GS_TRY(rec_pass_pits(p, step, lsink, np1));
             GS_CUDA(cudaStreamSynchronize(p->stream));
+            if (solving) GS_TRY(flow_status(p, *sweep_st));
+            solving = false;
             int flags = 0;
             bool anybig = false, allbig = true;
             for (int m = 0; m < nm; m++) {
@@ -395,9 +402,11 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
                 // receivers and the surface order do not need the flat BFS;
                 // the flat routing and the order's ties do: join it between
                 GS_TRY(receivers(p, p->R, 1.1, surf, sealevel, p->gid, p->rcv, p->dist, p->wgt, p->rslot));
-                // the water surface differs from h only on lakes: reuse h's order
-                GS_TRY(flow_order_from(p, surf, h, p->order_i, p->order));
-                GS_TRY(flow_order_ties_prepare(p));
+                if (flow_needs_order(p)) {
+                    // the water surface differs from h only on lakes: reuse h's order
+                    GS_TRY(flow_order_from(p, surf, h, p->order_i, p->order));
+                    GS_TRY(flow_order_ties_prepare(p));
+                }
                 launch(p, k_div, G, B, (int64_t)n, (const double*)p->nfa, dt, p->q2);
                 launch(p, k_chunk_sum, p->nchunk, 256, (const int*)p->chunk_lo, (const double*)p->q2,
                        p->chunk_part);
@@ -413,7 +422,11 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
                     launch(p, k_lsink_keep, G, B, n, (const int*)p->vmember, (const uint8_t*)p->mbig,
                            (const uint8_t*)p->lsink_prev, lsink);
                 GS_TRY(rec_pass_rebuild(p, step, surf));
-                GS_TRY(flow_order_ties(p, p->pdir, p->order));
+                if (flow_needs_order(p)) GS_TRY(flow_order_ties(p, p->pdir, p->order));
+                // the graph is prepared before the residual is read: one
+                // synchronisation gives the residual and the check
+                GS_TRY(flow_prepare(p, TG_CASCADE, p->rcv, p->wgt, p->rslot, p->q, surf, p->pdir, p->order,
+                                    p->h_pinned));
                 GS_CUDA(cudaStreamSynchronize(p->stream));
                 bool anysolve = false, allsolve = true;
                 for (int m = 0; m < nm; m++) {
@@ -427,11 +440,12 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
                         launch(p, k_rhs_members, G, B, n, (const int*)p->vmember, (const uint8_t*)p->msolve,
                                p->q2);
                     }
-                    // solve into FA's buffer: FA is consumed already
-                    GS_TRY(flow_prepare(p, p->rcv, p->wgt, p->rslot, p->q, p->order, p->h_pinned));
-                    GS_CUDA(cudaStreamSynchronize(p->stream));
+                    // solve into FA's buffer: FA is consumed already; the
+                    // sweep's status is read at the next synchronisation
                     const int ok_c = p->h_pinned[0] ? 0 : 1;
-                    GS_TRY(flow_run(p, p->rcv, p->wgt, p->rslot, p->q2, p->q, &cyc, p->order, ok_c, nullptr));
+                    GS_TRY(flow_run(p, TG_CASCADE, p->rcv, p->wgt, p->rslot, p->q2, p->q, &cyc, p->order, ok_c,
+                                    sweep_st));
+                    solving = true;
                     GS_TRY(rec_pass_solve(p, step, p->order, ok_c, p->q));
                     total_cycles += cyc;
                     launch(p, k_cascade_accum, G, B, n, (const double*)p->q, dt, h, (const double*)p->wf,
@@ -457,6 +471,10 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
                     act[m] = 0;
                 }
             }
+        }
+        if (solving) {   // the loop ended right after a solve (pass limit, stagnation)
+            GS_CUDA(cudaStreamSynchronize(p->stream));
+            GS_TRY(flow_status(p, *sweep_st));
         }
         launch(p, k_lake_zero, G, B, n, h, (const double*)p->wf, (const int*)pit_ids, (const int*)p->vmember,
                (const uint8_t*)p->mlakes, fal);

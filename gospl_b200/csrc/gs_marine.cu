@@ -791,7 +791,7 @@ int sea_change(gs_plan* p, double* h, double* cum_ed, double* eb, const double* 
         double* t2 = tmpb;
         launch(p, k_marine_g, G, B, n, (const double*)hl, sealevel, gmar, G_);
         GS_LAUNCH();
-        GS_TRY(flow_order(p, fz, p->order));
+        GS_TRY(marine_prepare(p, cand, wgt, fz, p->order));
         // r0 = G dt/A S[dep / dt]
         launch(p, k_marine_scale, G, B, n, 1.0 / dt, (const double*)vdep, (const double*)nullptr, t1);
         GS_LAUNCH();

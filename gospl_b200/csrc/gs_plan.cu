@@ -55,6 +55,7 @@ static void plan_free(gs_plan* p) {
     p->prof_ev.clear();
     free_members(p);
     record_free(p);
+    tiles_free(p);
     if (p->side_a) cudaStreamDestroy(p->side_a);
     if (p->side_b) cudaStreamDestroy(p->side_b);
     if (p->h_pinned) cudaFreeHost(p->h_pinned);
@@ -124,16 +125,25 @@ int plan_create(int64_t nb, const int32_t* nnb, const int32_t* ngb, const double
             h_vd[(size_t)s * n + i] = vdist[(size_t)i * 12 + s];
         }
     }
+    bool mutual = true;   // every edge is listed by both of its ends
     for (int i = 0; i < n; i++) {
-        int slots[12], cnt = 0;
+        int slots[12], ids[12], cnt = 0;
         for (int s = 0; s < nnb[i]; s++) {
-            int j = ngb[(size_t)i * 12 + s];
+            const int j = ngb[(size_t)i * 12 + s];
             if (j < 0 || j >= n) continue;
-            slots[cnt++] = s;
-            for (int t = 0; t < nnb[j]; t++)
-                if (ngb[(size_t)j * 12 + t] == i) { h_rev[(size_t)s * n + i] = (int8_t)t; break; }
+            int at = cnt++;   // insertion by ascending id
+            for (; at > 0 && ids[at - 1] > j; at--) {
+                ids[at] = ids[at - 1];
+                slots[at] = slots[at - 1];
+            }
+            ids[at] = j;
+            slots[at] = s;
+            const int32_t* row = ngb + (size_t)j * 12;
+            int t = 0;
+            while (t < nnb[j] && row[t] != i) t++;
+            if (t < nnb[j]) h_rev[(size_t)s * n + i] = (int8_t)t;
+            else mutual = false;
         }
-        std::sort(slots, slots + cnt, [&](int a, int b) { return ngb[(size_t)i * 12 + a] < ngb[(size_t)i * 12 + b]; });
         unsigned long long o = ~0ULL;
         for (int q = cnt - 1; q >= 0; q--) o = (o << 4) | (unsigned long long)slots[q];
         h_sorder[i] = o;
@@ -292,6 +302,8 @@ int plan_create(int64_t nb, const int32_t* nnb, const int32_t* ngb, const double
             goto fail;
         }
     }
+    st = mutual ? tiles_setup(p, nnb, ngb) : GS_OK;
+    if (st != GS_OK) goto fail;
     {
         const int64_t st0[2] = {0, (int64_t)n};
         const double ma0[1] = {maxarea};

@@ -3,6 +3,7 @@
 #include <vector>
 
 #include "gs_common.cuh"
+#include "gs_tiles.cuh"
 
 struct gs_plan {
     int64_t n = 0;      // vertices
@@ -110,6 +111,26 @@ struct gs_plan {
     int* order2 = nullptr;
     int* pos = nullptr;
     double* c = nullptr;                 // SPL coefficients [R][n]
+
+    // mesh tiles of the dataflow sweeps (gs_tiles.cu); tl_nt = 0: ordered sweeps
+    int tl_nt = 0;                       // tiles, one resident block each
+    int tl_T = 0;                        // vertices per tile
+    int tl_np = 0;                       // predecessor slots of a record (6, 8 or 12)
+    int tl_cap = 0;                      // most cut edges of a tile
+    int tl_par = 0;                      // half of tl_xb the next solve publishes in
+    int tl_dirty = 0;                    // tl_xb and the status word need a reset
+    size_t tl_smem = 0;
+    char* tl_pool = nullptr;             // the allocation that holds all of the following
+    int* tl_perm = nullptr;              // tile-major position -> vertex (null: identity)
+    int* tl_loc = nullptr;               // vertex -> position (null: identity)
+    int* tl_cut0 = nullptr;              // [tl_nt + 1] first cut edge of each tile
+    unsigned* tl_cut_q = nullptr;        // position across each cut edge
+    unsigned* tl_cut_l = nullptr;        // local vertex | slot << 16 of each cut edge
+    uint16_t* tl_cut_idx = nullptr;      // [W][n] by position: cut edge of each slot within its tile
+    int tl_full = 0;                     // the whole records of a tile fit its block's shared memory
+    double* tl_xb = nullptr;             // [2][n] values published between tiles, two solves in turn
+    unsigned* tl_status = nullptr;
+    gs::TileGraph tl_graph[gs::TG_N];
 
     // pit filling
     int8_t* ledge = nullptr;
@@ -258,9 +279,6 @@ int flow_direction_post(gs_plan* p, const double* h, bool down, const double* lf
 // lsink / sea masks for flow_direction(..., lsink = nullptr) graphs
 int sea_mask(gs_plan* p, const double* lfill, double sl, uint8_t* sea);
 int sink_mask(gs_plan* p, const double* wgt, const uint8_t* sea, uint8_t* lsink);
-int flow_solve(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot,
-               const double* b, double* x, int* cycle_nodes, const double* surface, const int* pdir,
-               int* order);
 int receivers_adjoint(gs_plan* p, const double* z, double sl, const int8_t* rslot, const double* gw, double* gself,
                       double* gnb, double* gz);
 int spl_adjoint(gs_plan* p, const double* hold, const double* s, const double* fal, const double* rain,
@@ -284,7 +302,8 @@ int adjoint_step(gs_plan* p, int slot, double* lam, const double* rain, double k
                  double* gK, double* gU, double* grain, double* gbl);
 int hillslope_adjoint(gs_plan* p, const double* h_in, double* lam, double sealevel, double cda, double cdm,
                       double dt, double rtol, int max_iter, int* iters);
-int sweep_flow_adjoint(gs_plan* p, const int* rcv, const double* wgt, const int* order, const double* g, double* y);
+int sweep_flow_adjoint(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const int* order,
+                       const double* g, double* y);
 int sweep_spl_adjoint(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const double* c,
                       const int* order, const double* g, double* y);
 int spl_sweep(gs_plan* p, const int* rcv, const double* c, const int8_t* rslot, const double* hold,
@@ -307,8 +326,9 @@ int flow_order_from(gs_plan* p, const double* surface, const double* base_surfac
                     int* order);
 int flow_order_ties_prepare(gs_plan* p);   // after flow_order: tie groups of the surface
 int flow_order_ties(gs_plan* p, const int* pdir, int* order);   // after prepare: ties by pdir
-int flow_prepare(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, double* x, const int* order,
-                 int* bad_host);
+bool flow_needs_order(const gs_plan* p);   // the flow sweeps run in a vertex order (else on tiles)
+int flow_prepare(gs_plan* p, int graph, const int* rcv, const double* wgt, const int8_t* rslot, double* x,
+                 const double* z, const int* pdir, const int* order, int* bad_host);
 // status_host (pinned): when given, the ordered sweep's status is copied
 // there asynchronously and the caller checks it after its next
 // synchronisation of the plan's stream; otherwise flow_run synchronises
@@ -325,9 +345,10 @@ int gm_axpby(gs_plan* p, int n, double a, const double* x, double b, const doubl
 // Marine flow accumulation q = (I - W^T)^-1 b over the marine receivers
 // (bit sets cand over the neighbour slots, weights w), donors summed in
 // ascending id, in the order of the marine surface (descending).
+int marine_prepare(gs_plan* p, const unsigned short* cand, const double* w, const double* z, int* order);
 int sweep_marine(gs_plan* p, const unsigned short* cand, const double* w, const int* order, const double* b,
                  double* q);
-int flow_run(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const double* b,
+int flow_run(gs_plan* p, int graph, const int* rcv, const double* wgt, const int8_t* rslot, const double* b,
              double* x, int* cycle_nodes, int* order, int ok, int* status_host);
 int group_sum_by_pit(gs_plan* p, const int* pit_ids, const uint8_t* mask, const double* vals,
                      double* out, int npits);
@@ -377,8 +398,7 @@ __global__ void k_cg_coop(int n, const int* __restrict__ nbr, const int8_t* __re
 int set_members(gs_plan* p, int nmem, const int64_t* start, const double* maxarea);
 int plan_tune(gs_plan* p, int knob, int value);
 int precision_buffers(gs_plan* p);
-int build_donors(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot);
-int spl_order(gs_plan* p);
+int sweeps_prepare(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const double* c);
 int sweep_flow_rhs(gs_plan* p, const double* wgt, const int* order, const double* b, double* x);
 int sweep_spl_rhs(gs_plan* p, const int* rcv, const double* c, const int* order2, const double* rhs, double* x);
 int flow_refine32(gs_plan* p, const double* wgt, const double* b, double* x, const int* order);

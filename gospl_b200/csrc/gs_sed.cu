@@ -741,8 +741,15 @@ int sed_change(gs_plan* p, double* h, double* cum_ed, const double* eb, const do
     int cyc = 0, total_cycles = 0;
     launch(p, k_sed_rhs, G, B, n, eb, (const double*)p->larea, p->q2);
     GS_LAUNCH();
-    GS_TRY(flow_prepare(p, rcv_i, wgt_i, p->rslot_i, vsed, p->order_i, p->h_pinned + 3));
-    GS_TRY(flow_run(p, rcv_i, wgt_i, p->rslot_i, p->q2, vsed, &cyc, p->order_i, p->order_i_valid, nullptr));
+    GS_TRY(flow_prepare(p, TG_CASCADE, rcv_i, wgt_i, p->rslot_i, vsed, nullptr, nullptr, p->order_i,
+                        p->h_pinned + 3));
+    int ok_i = p->order_i_valid;
+    if (!flow_needs_order(p)) {
+        // (tiles: edges outside the checked snapshot graph take the counter-based sweep)
+        GS_CUDA(cudaStreamSynchronize(p->stream));
+        ok_i = ok_i && !p->h_pinned[3];
+    }
+    GS_TRY(flow_run(p, TG_CASCADE, rcv_i, wgt_i, p->rslot_i, p->q2, vsed, &cyc, p->order_i, ok_i, nullptr));
     total_cycles += cyc;
     // lsinki: sinks of the snapshot graph (flowplex.py:785-791)
     GS_TRY(sink_mask(p, wgt_i, sea, lsink));
@@ -776,6 +783,7 @@ int sed_change(gs_plan* p, double* h, double* cum_ed, const double* eb, const do
     };
     int step = 0, solves = 0;
     bool rebuilt = false;
+    int ok_c = 0;   // the last rebuilt graph passed its check
     while (any(act) && step < 5000) {
         GS_CUDA(cudaMemcpyAsync(p->mact, act.data(), nm, cudaMemcpyHostToDevice, p->stream));
         launch(p, k_sed_csink, G, B, n, (const uint8_t*)lsink, (const int*)pit_ids, (const uint8_t*)mout,
@@ -822,15 +830,22 @@ int sed_change(gs_plan* p, double* h, double* cum_ed, const double* eb, const do
                 const double* surf = (step == 100) ? lfill : sfill;
                 rebuilt = true;
                 GS_TRY(receivers(p, p->R, 1.1, surf, sealevel, p->gid, p->rcv, p->dist, p->wgt, p->rslot));
-                GS_TRY(flow_order_from(p, surf, hl, p->order_i, p->order));
-                GS_TRY(flow_order_ties_prepare(p));
+                if (flow_needs_order(p)) {
+                    GS_TRY(flow_order_from(p, surf, hl, p->order_i, p->order));
+                    GS_TRY(flow_order_ties_prepare(p));
+                }
                 GS_TRY(fill_join(p, st));
                 GS_TRY(flow_direction_post(p, surf, true, lfill, pit_ids, flat_dirs, sealevel, p->rcv, p->dist,
                                            p->wgt, p->rslot, lsink, sea_s));
                 if (!every)
                     launch(p, k_lsink_keep, G, B, n, (const int*)p->vmember, (const uint8_t*)p->mbig,
                            (const uint8_t*)p->lsink_prev, lsink);
-                GS_TRY(flow_order_ties(p, p->pdir, p->order));
+                // the tile graph is built with the rebuild (and kept over the
+                // passes that do not rebuild); its check comes back with the excess
+                if (flow_needs_order(p)) GS_TRY(flow_order_ties(p, p->pdir, p->order));
+                else
+                    GS_TRY(flow_prepare(p, TG_CASCADE, p->rcv, p->wgt, p->rslot, routed, surf, p->pdir, p->order,
+                                        p->h_pinned));
             }
             // excess of each member (tmp.sum() > 0.5 maxarea, sedplex.py:349)
             launch(p, k_chunk_sum, p->nchunk, 256, (const int*)p->chunk_lo, (const double*)nv, p->chunk_part);
@@ -839,15 +854,19 @@ int sed_change(gs_plan* p, double* h, double* cum_ed, const double* eb, const do
             GS_LAUNCH();
             GS_CUDA(cudaMemcpyAsync(p->h_mresid, p->mresid, sizeof(double) * nm, cudaMemcpyDeviceToHost, p->stream));
             GS_CUDA(cudaStreamSynchronize(p->stream));
+            if (any(rebuild)) ok_c = p->h_pinned[0] ? 0 : 1;
             for (int m = 0; m < nm; m++) solve[m] = (big[m] && p->h_mresid[m] > 0.5 * p->mmaxarea[m]) ? 1 : 0;
             if (any(solve)) {
                 GS_CUDA(cudaMemcpyAsync(p->msolve, solve.data(), nm, cudaMemcpyHostToDevice, p->stream));
                 if (!all(solve))
                     launch(p, k_rhs_members, G, B, n, (const int*)p->vmember, (const uint8_t*)p->msolve, nv);
-                GS_TRY(flow_prepare(p, p->rcv, p->wgt, p->rslot, routed, p->order, p->h_pinned));
-                GS_CUDA(cudaStreamSynchronize(p->stream));
-                const int ok = p->h_pinned[0] ? 0 : 1;
-                GS_TRY(flow_run(p, p->rcv, p->wgt, p->rslot, nv, routed, &cyc, p->order, ok, nullptr));
+                if (flow_needs_order(p)) {
+                    GS_TRY(flow_prepare(p, TG_CASCADE, p->rcv, p->wgt, p->rslot, routed, nullptr, nullptr, p->order,
+                                        p->h_pinned));
+                    GS_CUDA(cudaStreamSynchronize(p->stream));
+                    ok_c = p->h_pinned[0] ? 0 : 1;
+                }
+                GS_TRY(flow_run(p, TG_CASCADE, p->rcv, p->wgt, p->rslot, nv, routed, &cyc, p->order, ok_c, nullptr));
                 total_cycles += cyc;
                 GS_TRY(led_sum(p, n, nv, nullptr, nullptr, 1.0, GS_LED_ROUTED));
                 GS_TRY(led_cells(p, routed, p->wgt, lsink, pit_ids, mout));

@@ -358,8 +358,7 @@ static int coupled_ed(gs_plan* p, const double* hold, const double* fal, const u
     double* a = y2 + n;
     launch(p, k_fdep, G, B, n, p->fdepa, (const double*)p->larea, fal, sea, (const uint8_t*)p->outlet, p->flat, f);
     GS_LAUNCH();
-    GS_TRY(build_donors(p, rcv_i, wgt_i, p->rslot_i));
-    GS_TRY(spl_order(p));
+    GS_TRY(sweeps_prepare(p, rcv_i, wgt_i, p->rslot_i, p->c));
     EdSolve op(p, n, rcv_i, wgt_i, (const double*)p->c, (const double*)f, dt, t1, u, w, y2);
     // x0 = M^-1 hOld (detachment-limited), a = x0 + B hOld
     GS_TRY(sweep_spl_rhs(p, rcv_i, p->c, p->order2, hold, x));
@@ -373,6 +372,15 @@ static int coupled_ed(gs_plan* p, const double* hold, const double* fal, const u
     const int st = gmres_solve(p, op, a, x, 1.0e-13, 200, &applies, &relres);
     p->ed_iters = applies;
     p->ed_relres = relres;
+    if (p->tl_nt > 0) {
+        // the sweeps were only queued: one that stopped explains a failure
+        const int sw = tile_status(p, "transport-limited SPL: a sweep did not complete");
+        if ((unsigned)sw == TILE_REJECTED) {
+            set_error(GS_EINVAL, "transport-limited SPL: the receivers are not those of the last flow accumulation");
+            return GS_EINVAL;
+        }
+        GS_TRY(sw);
+    }
     if (st == GS_EMAXITER) {
         set_error(GS_EMAXITER, "transport-limited SPL: GMRES did not converge");
         return GS_EMAXITER;

@@ -913,6 +913,12 @@ static int order_by_surface(gs_plan* p, const double* z, int* order) {
     return GS_OK;
 }
 
+// Breaking the surface ties of order_by_surface by flat distance descending
+// (ties of both by vertex id): only the members of tie groups are re-sorted,
+// by (group start, ~(pdir + 1)), and written back to their positions.  Gives
+// the order of a stable sort by (surface desc, pdir desc).  The tie groups
+// depend on the surface only (order_ties_prepare, which reads their count back
+// to the host); the flat distances are needed only by order_ties_finish.
 static int order_ties_prepare(gs_plan* p) {
     const int n = (int)p->n;
     const int B = 256, G = grid_for(n, B);
@@ -982,17 +988,6 @@ static int order_ties_finish(gs_plan* p, const int* pdir, int* order) {
     launch(p, k_tie_scatter, grid_for(m, B), B, m, (const int*)cpos, (const int*)cval2, order);
     GS_LAUNCH();
     return GS_OK;
-}
-
-// Breaks the surface ties of order_by_surface by flat distance descending
-// (ties of both by vertex id): only the members of tie groups are re-sorted,
-// by (group start, ~(pdir + 1)), and written back to their positions.  Gives
-// the order of a stable sort by (surface desc, pdir desc).  The tie groups
-// depend on the surface only (order_ties_prepare, which reads their count back
-// to the host); the flat distances are needed only by order_ties_finish.
-static int order_ties(gs_plan* p, const int* pdir, int* order) {
-    GS_TRY(order_ties_prepare(p));
-    return order_ties_finish(p, pdir, order);
 }
 
 // Checks that every weighted edge goes forward in `order`; the result
@@ -1130,13 +1125,28 @@ static int ordered_status(gs_plan* p, int* st) {
     return GS_OK;
 }
 
-// Everything of an ordered flow sweep that does not need b, for an order
-// built by flow_order (+ flow_order_ties): its check (result in *bad_host once
-// the stream reaches it), the donor masks and the sentinel-filled output.
-int flow_prepare(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, double* x, const int* order,
-                 int* bad_host) {
+// The tile dataflow (gs_tiles.cu) solves the FP64 sweeps of every plan whose
+// tiles fit; the ordered sweeps remain for larger meshes and for the FP32
+// sweeps of the precision form, and only they need an order.
+bool flow_needs_order(const gs_plan* p) { return p->tl_nt == 0 || p->fp32; }
+
+// Everything of a flow sweep that does not need b: the tile records (with the
+// acyclicity check on the surface z and the flat distances) or, for an order
+// built by flow_order (+ flow_order_ties), its check, the donor masks and the
+// sentinel-filled output.  The check's result is in *bad_host once the stream
+// reaches it.
+int flow_prepare(gs_plan* p, int graph, const int* rcv, const double* wgt, const int8_t* rslot, double* x,
+                 const double* z, const int* pdir, const int* order, int* bad_host) {
     const int n = (int)p->n;
     if (n == 0) return GS_OK;
+    if (!flow_needs_order(p)) {
+        GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));
+        // without a surface the edges must be those of the checked snapshot graph
+        GS_TRY(tile_build(p, graph, true, false, rcv, wgt, rslot, z, pdir, z ? nullptr : p->tl_graph[TG_SNAP].pm,
+                          p->i_scalar + 14));
+        GS_CUDA(cudaMemcpyAsync(bad_host, p->i_scalar + 14, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+        return GS_OK;
+    }
     GS_TRY(order_check_async(p, rcv, wgt, order, bad_host));
     GS_CUDA(cudaMemsetAsync(p->don_mask, 0, sizeof(uint32_t) * n, p->stream));
     GS_CUDA(cudaMemsetAsync(p->don_k, 0, sizeof(unsigned long long) * n, p->stream));
@@ -1149,13 +1159,18 @@ int flow_prepare(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rs
 
 // The sweep proper, after flow_prepare: the ordered kernel when the order is
 // valid (ok), else the counter-based dataflow solve.
-int flow_run(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const double* b, double* x,
-             int* cycle_nodes, int* order, int ok, int* status_host) {
+int flow_run(gs_plan* p, int graph, const int* rcv, const double* wgt, const int8_t* rslot, const double* b,
+             double* x, int* cycle_nodes, int* order, int ok, int* status_host) {
     const int n = (int)p->n;
     *cycle_nodes = 0;
     if (status_host) *status_host = 0;
     if (n == 0) return GS_OK;
     if (!ok) return flow_solve_counted(p, rcv, wgt, rslot, b, x, cycle_nodes);
+    if (!flow_needs_order(p)) {
+        GS_TRY(tile_solve(p, graph, false, b, x, nullptr));
+        if (status_host) return tile_status_async(p, status_host);   // checked by the caller (flow_status)
+        return tile_status(p, "flow sweep did not complete");
+    }
     if (p->fp32) return flow_refine32(p, wgt, b, x, order);
     GS_CUDA(cudaMemsetAsync(p->ctr, 0, sizeof(unsigned) * 8, p->stream));
     FlowOrd op{n, p->nbr, p->don_mask, p->don_k, p->sorder, wgt, b, x};
@@ -1173,23 +1188,6 @@ int flow_run(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot,
         return st;
     }
     return GS_OK;
-}
-
-int flow_solve(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const double* b, double* x,
-               int* cycle_nodes, const double* surface, const int* pdir, int* order) {
-    const int n = (int)p->n;
-    *cycle_nodes = 0;
-    if (n == 0) return GS_OK;
-    int ok = 0;
-    if (surface) {
-        GS_TRY(order_by_surface(p, surface, order));
-        if (pdir) GS_TRY(order_ties(p, pdir, order));
-        GS_TRY(flow_prepare(p, rcv, wgt, rslot, x, order, p->h_pinned));
-        GS_CUDA(cudaStreamSynchronize(p->stream));
-        ok = p->h_pinned[0] ? 0 : 1;
-    }
-    if (order == p->order_i) p->order_i_valid = ok;
-    return flow_run(p, rcv, wgt, rslot, b, x, cycle_nodes, order, ok, nullptr);
 }
 
 // SPL edges i -> rcv (c != 0) run against the flow order: need pos[rcv] > pos[i]
@@ -1210,6 +1208,17 @@ int spl_sweep(gs_plan* p, const int* rcv, const double* c, const int8_t* rslot, 
     if (n == 0) return GS_OK;
     const int ok = reuse_order && p->order_i_valid;
     if (!ok) return spl_sweep_counted(p, rcv, c, rslot, hold, s, cycle_nodes);
+    if (!flow_needs_order(p)) {
+        // receivers first; every edge must be one of the checked snapshot
+        // graph, else the sweep stops at once and the counter-based one runs
+        GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));
+        GS_TRY(tile_build(p, TG_UP, false, true, rcv, c, rslot, nullptr, nullptr, p->tl_graph[TG_SNAP].pm,
+                          p->i_scalar + 14));
+        GS_TRY(tile_solve(p, TG_UP, true, hold, s, p->i_scalar + 14));
+        const int st = tile_status(p, "SPL sweep did not complete");
+        if ((unsigned)st == TILE_REJECTED) return spl_sweep_counted(p, rcv, c, rslot, hold, s, cycle_nodes);
+        return st;
+    }
     // the check of the order against the SPL edges is read by the sweep
     // itself (no host round trip): a rejected order stops it at once and the
     // counter-based sweep runs instead
@@ -1243,10 +1252,28 @@ int spl_sweep(gs_plan* p, const int* rcv, const double* c, const int8_t* rslot, 
     return GS_OK;
 }
 
+// the marine graph of the surface z (receivers strictly lower) for
+// sweep_marine: tile records, or the surface order
+int marine_prepare(gs_plan* p, const unsigned short* cand, const double* w, const double* z, int* order) {
+    if (p->n == 0) return GS_OK;
+    if (p->tl_nt == 0) return flow_order(p, z, order);
+    GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));
+    return tile_build_marine(p, TG_CASCADE, cand, w, z, p->i_scalar + 14);
+}
+
 int sweep_marine(gs_plan* p, const unsigned short* cand, const double* w, const int* order, const double* b,
                  double* q) {
     const int n = (int)p->n;
     if (n == 0) return GS_OK;
+    if (p->tl_nt > 0) {
+        GS_TRY(tile_solve(p, TG_CASCADE, false, b, q, p->i_scalar + 14));
+        const int st = tile_status(p, "marine sweep did not complete");
+        if ((unsigned)st == TILE_REJECTED) {
+            set_error(GS_EINVAL, "marine sweep: the marine receivers are not below their donors in the surface order");
+            return GS_EINVAL;
+        }
+        return st;
+    }
     launch(p, k_positions, grid_for(n, 256), 256, n, order, p->pos);
     GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));
     launch(p, k_check_marine_order, grid_for(n, 256), 256, n, (const int*)p->nbr, (const int8_t*)p->nnb, cand,
@@ -1273,9 +1300,16 @@ int sweep_marine(gs_plan* p, const unsigned short* cand, const double* w, const 
 }
 
 // y = (I - W)^-1 g over the graph rcv/wgt whose valid flow order is `order`
-int sweep_flow_adjoint(gs_plan* p, const int* rcv, const double* wgt, const int* order, const double* g, double* y) {
+int sweep_flow_adjoint(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const int* order,
+                       const double* g, double* y) {
     const int n = (int)p->n;
     if (n == 0) return GS_OK;
+    if (p->tl_nt > 0) {
+        GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));
+        GS_TRY(tile_build(p, TG_UP, false, false, rcv, wgt, rslot, nullptr, nullptr, nullptr, p->i_scalar + 14));
+        GS_TRY(tile_solve(p, TG_UP, false, g, y, nullptr));
+        return tile_status(p, "adjoint flow sweep did not complete");
+    }
     launch(p, k_reverse, grid_for(n, 256), 256, n, order, p->order2);
     GS_CUDA(cudaMemsetAsync(p->ctr, 0, sizeof(unsigned) * 8, p->stream));
     launch(p, k_fill_sent, grid_for(n, 256), 256, n, y);
@@ -1301,6 +1335,12 @@ int sweep_spl_adjoint(gs_plan* p, const int* rcv, const double* wgt, const int8_
     GS_CUDA(cudaMemsetAsync(p->don_k, 0, sizeof(unsigned long long) * n, p->stream));
     launch(p, k_flow_donors, grid_for(n, 256), 256, n, p->R, rcv, wgt, rslot, (const int8_t*)p->rev, p->don_mask,
            p->don_k);
+    if (p->tl_nt > 0) {
+        GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));
+        GS_TRY(tile_build(p, TG_CASCADE, true, true, rcv, c, rslot, nullptr, nullptr, nullptr, p->i_scalar + 14));
+        GS_TRY(tile_solve(p, TG_CASCADE, true, g, y, nullptr));
+        return tile_status(p, "adjoint SPL sweep did not complete");
+    }
     GS_CUDA(cudaMemsetAsync(p->ctr, 0, sizeof(unsigned) * 8, p->stream));
     launch(p, k_fill_sent, grid_for(n, 256), 256, n, y);
     SplAdjOrd op{n, p->R, p->nbr, p->don_mask, p->don_k, p->sorder, c, g, y};
@@ -1485,10 +1525,10 @@ int spl_refine32(gs_plan* p, const int* rcv, const double* c, const double* hold
 
 // Plain FP64 sweeps with caller-given right-hand sides, for solvers that
 // apply the flow or SPL inverse repeatedly (the coupled erosion-deposition
-// system).  sweep_flow_rhs needs the donor masks of the graph (flow_prepare or
-// build_donors) and a valid flow order; sweep_spl_rhs the receivers-first
-// order (the flow order reversed).
-int build_donors(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot) {
+// system), after sweeps_prepare on the snapshot graph rcv/wgt/rslot and the
+// SPL coefficients c.  On tiles the sweeps are only queued: their status is
+// read at the end of the solver (tile_status).
+static int build_donors(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot) {
     const int n = (int)p->n;
     GS_CUDA(cudaMemsetAsync(p->don_mask, 0, sizeof(uint32_t) * n, p->stream));
     GS_CUDA(cudaMemsetAsync(p->don_k, 0, sizeof(unsigned long long) * n, p->stream));
@@ -1500,6 +1540,7 @@ int build_donors(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rs
 
 int sweep_flow_rhs(gs_plan* p, const double* wgt, const int* order, const double* b, double* x) {
     const int n = (int)p->n;
+    if (p->tl_nt > 0) return tile_solve(p, TG_CASCADE, false, b, x, p->i_scalar + 14);
     GS_CUDA(cudaMemsetAsync(p->ctr, 0, sizeof(unsigned) * 8, p->stream));
     launch(p, k_fill_sent, grid_for(n, 256), 256, n, x);
     FlowOrd op{n, p->nbr, p->don_mask, p->don_k, p->sorder, wgt, b, x};
@@ -1516,6 +1557,7 @@ int sweep_flow_rhs(gs_plan* p, const double* wgt, const int* order, const double
 
 int sweep_spl_rhs(gs_plan* p, const int* rcv, const double* c, const int* order2, const double* rhs, double* x) {
     const int n = (int)p->n;
+    if (p->tl_nt > 0) return tile_solve(p, TG_UP, true, rhs, x, p->i_scalar + 14);
     GS_CUDA(cudaMemsetAsync(p->ctr, 0, sizeof(unsigned) * 8, p->stream));
     launch(p, k_fill_sent, grid_for(n, 256), 256, n, x);
     SplOrd op{n, p->R, rcv, c, rhs, x};
@@ -1530,9 +1572,17 @@ int sweep_spl_rhs(gs_plan* p, const int* rcv, const double* c, const int* order2
     return GS_OK;
 }
 
-// order2 = the snapshot flow order reversed (receivers first)
-int spl_order(gs_plan* p) {
+int sweeps_prepare(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const double* c) {
     const int n = (int)p->n;
+    if (p->tl_nt > 0) {
+        // edges outside the checked snapshot graph stop the sweeps (i_scalar[14])
+        const uint16_t* ref = p->tl_graph[TG_SNAP].pm;
+        GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));
+        GS_TRY(tile_build(p, TG_CASCADE, true, false, rcv, wgt, rslot, nullptr, nullptr, ref, p->i_scalar + 14));
+        return tile_build(p, TG_UP, false, true, rcv, c, rslot, nullptr, nullptr, ref, p->i_scalar + 14);
+    }
+    GS_TRY(build_donors(p, rcv, wgt, rslot));
+    // order2 = the snapshot flow order reversed (receivers first)
     launch(p, k_reverse, grid_for(n, 256), 256, n, (const int*)p->order_i, p->order2);
     GS_LAUNCH();
     return GS_OK;
