@@ -686,6 +686,7 @@ __global__ void __launch_bounds__(BFT_THREADS, 2) k_bfs_tiles(int M, int S, int 
     __shared__ int s_over[3];
     __shared__ int s_pmin;
     __shared__ int s_nx;
+    __shared__ int s_pt;
     const int ntiles = (M + T - 1) / T;
     int* gmin = ctl;               // [3] smallest pending distance after rounds r % 3
     int* pend = ctl + 3;           // [ntiles] smallest pending distance of each tile
@@ -711,8 +712,12 @@ __global__ void __launch_bounds__(BFT_THREADS, 2) k_bfs_tiles(int M, int S, int 
         int* gnext = gmin + ((r + 1) % 3);
         if (blockIdx.x == 0 && tid == 0) gmin[(r + 2) % 3] = INF;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+            // one thread reads the tile's pending minimum for the block: other
+            // blocks lower it meanwhile, and all threads must take one branch
             __syncthreads();
-            const int pt = ((volatile int*)pend)[t];
+            if (tid == 0) s_pt = ((volatile int*)pend)[t];
+            __syncthreads();
+            const int pt = s_pt;
             if (pt > hi) {
                 // nothing of this window here: its pending minimum stays for later
                 if (tid == 0 && pt != INF) atomicMin(gnext, pt);
@@ -1371,7 +1376,9 @@ static int bfs_tiles(gs_plan* p, int M, int S, const int* rows, int* ld) {
     int* ctl = p->front1;
     int* depth = p->i_scalar + 4;
     int* rounds = p->i_scalar + 15;
-    int window = p->bfs_window;
+    // the search over all depressions also comes here with the knob at 0, when
+    // the visited set is too large for one block
+    int window = p->bfs_window > 0 ? p->bfs_window : 64;
     void* args[] = {(void*)&m, (void*)&s, (void*)&t, (void*)&rows, (void*)&seeds, (void*)&nseed, (void*)&ld,
                     (void*)&ctl, (void*)&window, (void*)&depth, (void*)&rounds};
     cudaEvent_t stop = nullptr;
