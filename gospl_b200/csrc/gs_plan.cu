@@ -220,7 +220,8 @@ int plan_create(int64_t nb, const int32_t* nnb, const int32_t* ngb, const double
         TRYP(dalloc(&p->xe_u, (size_t)p->xe_cap));
         TRYP(dalloc(&p->xe_v, (size_t)p->xe_cap));
         TRYP(dalloc(&p->xe_w, (size_t)p->xe_cap));
-        TRYP(dalloc(&p->bfs_rows, (size_t)(((W + 1 + 3) / 4) * 4) * N));
+        // rows of the flat searches: a count and W ids, or 8 or 16 ids
+        TRYP(dalloc(&p->bfs_rows, (size_t)std::max(((W + 1 + 3) / 4) * 4, W <= 8 ? 8 : 16) * N));
         TRYP(dalloc(&p->comp, N));
         TRYP(dalloc(&p->minseed, N));
         TRYP(dalloc(&p->lab, N));

@@ -5,6 +5,17 @@
 #include "gs_common.cuh"
 #include "gs_tiles.cuh"
 
+namespace gs {
+// arguments of the flat pass of one fill (caller's arrays)
+struct FlatArgs {
+    double* lfill = nullptr;
+    const int* pit_ids = nullptr;
+    int* flat_dirs = nullptr;
+    const double* h = nullptr;
+    double sealevel = 0.0;
+};
+}  // namespace gs
+
 struct gs_plan {
     int64_t n = 0;      // vertices
     int W = 0;          // neighbour slots stored (max FVnNb)
@@ -198,7 +209,8 @@ struct gs_plan {
     cudaStream_t side_b = nullptr;
     cudaEvent_t ev_fork_a = nullptr, ev_a = nullptr, ev_fork_b = nullptr, ev_b = nullptr;
     int* h_pinned = nullptr;             // pinned host words [16]
-    int bfs_pending = 0;                 // flat BFS issued on side_b, not yet joined
+    int bfs_pending = 0;                 // flat pass issued on side_b, not yet joined (2: by depressions)
+    gs::FlatArgs flat_args;              // its arguments, for the join within the same call
 
     // flow / cascade
     double* nfa = nullptr;
