@@ -276,44 +276,100 @@ __global__ void k_mask_changed(int n, const double* __restrict__ h, double sl, c
 }
 
 // ---------------------------------------------------------------------------
-// The whole CG loop in one cooperative launch: three grid barriers per
-// iteration (after A p and its dot, after the update and its dots, after the
-// new direction), convergence decided on the device.  Dot products are block
-// partials in a fixed order; every block sums the partials of all blocks in
-// the same order (one warp, lane-strided, then a shuffle-down tree), so all
-// threads hold bitwise the same scalars and leave the loop together.
-__device__ __forceinline__ void block_sum2(double a, double b, double* out_a, double* out_b) {
-    __shared__ double sa[256], sb[256];
-    sa[threadIdx.x] = a;
-    sb[threadIdx.x] = b;
+// The whole CG loop in one cooperative launch: grid barriers between its
+// phases, convergence decided on the device.  Dot products are partial sums of
+// groups of 256 threads in a fixed order; every block adds the partials of all
+// groups in the same order (one warp, lane-strided, then a shuffle-down tree),
+// so all threads hold bitwise the same scalars and leave the loop together.
+// A block holds up to four groups: the sums depend on the number of groups
+// alone, and a grid barrier is met by one block per SM instead of four.
+// Latency bounds an iteration on small meshes: two grid barriers, each with
+// the partials' trip through L2, and the gathers of a row.  At 163,842 rows an
+// iteration takes 17 us, and 27 us with four blocks per SM, one load of the
+// partials after the other and one slot of a row after the other; the solve
+// of 2,621,442 rows from a guess that needs no iteration 0.097 and 0.15 ms.
+// Sums published in tagged words that every block polls, in place of the
+// barrier, took 20 to 23 us.
+constexpr int CG_GROUP = 256;
+constexpr int CG_GROUPS = 4;                 // groups per block at most
+constexpr int CG_MAXG = 160 * CG_GROUPS;     // groups in all at most (shared staging of their partials)
+constexpr int CG_SMEM = 2 * CG_GROUP * CG_GROUPS;   // doubles of shared memory, for either sum in turn
+static_assert(CG_SMEM >= 3 * CG_MAXG + 3, "the staged partials and totals have to fit");
+
+// groups of 256 threads of this block: pairwise tree (strides 128 to 1); the
+// first warp of each group finishes by shuffles, the same pairs as in memory
+// (thread 0 of the group gets them)
+__device__ __forceinline__ void group_sum2(double* sm, double a, double b, double* out_a, double* out_b) {
+    const int t = threadIdx.x & (CG_GROUP - 1);
+    double* pa = sm + (threadIdx.x - t);
+    double* pb = pa + CG_GROUP * CG_GROUPS;
+    pa[t] = a;
+    pb[t] = b;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            sa[threadIdx.x] += sa[threadIdx.x + s];
-            sb[threadIdx.x] += sb[threadIdx.x + s];
+    for (int s = CG_GROUP / 2; s > 32; s >>= 1) {
+        if (t < s) {
+            pa[t] += pa[t + s];
+            pb[t] += pb[t + s];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        *out_a = sa[0];
-        *out_b = sb[0];
+    if (t < 32) {
+        double u = pa[t] + pa[t + 32], v = pb[t] + pb[t + 32];
+        for (int o = 16; o > 0; o >>= 1) {
+            u += __shfl_down_sync(0xffffffffu, u, o);
+            v += __shfl_down_sync(0xffffffffu, v, o);
+        }
+        if (t == 0 && out_a) {
+            *out_a = u;
+            *out_b = v;
+        }
     }
     __syncthreads();
 }
 
-// sum over blocks of part[i * stride + off], identical in every block
-__device__ __forceinline__ double grid_total(const double* part, int stride, int off, int nb) {
-    __shared__ double tot;
+// NV sums over the groups of part[g * stride + off + v], identical in every
+// block: the partials staged in shared memory by all threads (one L2 latency),
+// then lane-strided additions by one warp and a shuffle-down tree
+template <int NV>
+__device__ __forceinline__ void grid_totals(double* sm, const double* part, int stride, int off, int ng,
+                                            double (&out)[NV]) {
+    double* tot = sm + 3 * CG_MAXG;
+    for (int i = threadIdx.x; i < ng * NV; i += blockDim.x)
+        sm[i] = __ldcg(part + (size_t)(i / NV) * stride + off + i % NV);
+    __syncthreads();
     if (threadIdx.x < 32) {
-        double acc = 0.0;
-        for (int i = threadIdx.x; i < nb; i += 32) acc += ((volatile const double*)part)[(size_t)i * stride + off];
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if (threadIdx.x == 0) tot = acc;
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            double acc = 0.0;
+            for (int i = threadIdx.x; i < ng; i += 32) acc += sm[i * NV + v];
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+            if (threadIdx.x == 0) tot[v] = acc;
+        }
     }
     __syncthreads();
-    double t = tot;
+#pragma unroll
+    for (int v = 0; v < NV; v++) out[v] = tot[v];
     __syncthreads();
-    return t;
+}
+
+// coefficients and neighbours of slots s0 to s0 + CG_SLOTS - 1 of row k, loaded
+// together; a slot past the row's, without a neighbour or with a zero
+// coefficient reads as coefficient 0 of the row itself
+constexpr int CG_SLOTS = 6;
+__device__ __forceinline__ void cg_slots(int n, int k, int s0, int deg, const double* __restrict__ coef,
+                                         const int* __restrict__ nbr, double (&o)[CG_SLOTS], int (&j)[CG_SLOTS]) {
+#pragma unroll
+    for (int t = 0; t < CG_SLOTS; t++) {
+        const bool has = s0 + t < deg;
+        o[t] = has ? coef[(size_t)(s0 + t + 1) * n + k] : 0.0;
+        j[t] = has ? nbr[(size_t)(s0 + t) * n + k] : -1;
+    }
+#pragma unroll
+    for (int t = 0; t < CG_SLOTS; t++)
+        if (j[t] < 0) {
+            o[t] = 0.0;
+            j[t] = k;
+        }
 }
 
 // Jacobi-PCG on the area-weighted symmetric form S = A (I + L) of the
@@ -326,22 +382,25 @@ __device__ __forceinline__ double grid_total(const double* part, int stride, int
 // its product: each thread forms p'_j = z_j + b p_j of the neighbours it
 // gathers (the same operations as a separate update pass, so the same bits)
 // and writes its own p'_k to the other buffer.  Two barriers per iteration;
-// block partial sums are added in block order by every block.  Fixed rows
-// (flat outlets, no area) keep x = x0.  Slots are unrolled to MAXW so the
-// gathers of a row issue together; <= 64 registers for four 256-thread
-// blocks per SM.
-__global__ void __launch_bounds__(256, 4) k_cg_coop(int n, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
+// group partial sums are added in group order by every block.  Fixed rows
+// (flat outlets, no area) keep x = x0.  The gathers of a row issue together in
+// batches of CG_SLOTS (with a branch on each slot they waited for one another).
+__global__ void __launch_bounds__(CG_GROUP * CG_GROUPS, 1) k_cg_coop(int n, int ng, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
                                                     const double* __restrict__ coef, const double* __restrict__ farea,
                                                     const uint8_t* __restrict__ fix, const double* __restrict__ x0,
                                                     double* x, double* b, double* r, double* z, double* p0, double* p1,
                                                     double* ap, double* part, double rtol, int max_iter, int* it_out,
                                                     double* res_out, const double* __restrict__ guess) {
     cg::grid_group grid = cg::this_grid();
-    const int nb = gridDim.x, blk = blockIdx.x;
-    const int gtid = blk * blockDim.x + threadIdx.x, gsz = nb * blockDim.x;
-    double* pc = part;             // initial dots [3 nb]
-    double* pa = part + 3 * nb;    // p.Ap [2 nb]
-    double* pb = part + 5 * nb;    // r.z, r.r [2 nb]
+    __shared__ double sm[CG_SMEM];
+    // group of this thread; a thread past the last group has no rows
+    const int grp = blockIdx.x + (threadIdx.x / CG_GROUP) * gridDim.x;
+    const bool in = grp < ng;
+    const int gtid = in ? grp * CG_GROUP + (threadIdx.x & (CG_GROUP - 1)) : n, gsz = ng * CG_GROUP;
+    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
+    double* pc = part;             // initial dots [3 ng]
+    double* pa = part + 3 * ng;    // p.Ap [2 ng]
+    double* pb = part + 5 * ng;    // r.z, r.r [2 ng]
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
     for (int k = gtid; k < n; k += gsz) {
         const double x0k = x0[k];
@@ -360,18 +419,23 @@ __global__ void __launch_bounds__(256, 4) k_cg_coop(int n, const int* __restrict
         const double ck = coef[k];
         double bk = x0k;
         double y = ck * xk;
+        for (int s0 = 0; s0 < deg; s0 += CG_SLOTS) {
+            double o[CG_SLOTS], xj[CG_SLOTS], gj[CG_SLOTS];
+            int j[CG_SLOTS];
+            uint8_t fj[CG_SLOTS];
+            cg_slots(n, k, s0, deg, coef, nbr, o, j);
 #pragma unroll
-        for (int s = 0; s < MAXW; s++) {
-            if (s < deg) {
-                const double o = coef[(size_t)(s + 1) * n + k];
-                const int j = nbr[(size_t)s * n + k];
-                if (o != 0.0 && j >= 0) {
-                    const double xj = x0[j];
-                    const double gj = guess ? guess[j] : xj;
-                    if (fix[j]) bk = bk - o * xj;
-                    else y = y + o * gj;
-                }
+            for (int t = 0; t < CG_SLOTS; t++) {
+                xj[t] = x0[j[t]];
+                gj[t] = guess ? guess[j[t]] : xj[t];
+                fj[t] = fix[j[t]];
             }
+#pragma unroll
+            for (int t = 0; t < CG_SLOTS; t++)
+                if (o[t] != 0.0) {
+                    if (fj[t]) bk = bk - o[t] * xj[t];
+                    else y = y + o[t] * gj[t];
+                }
         }
         const double fa = farea[k];
         bk = fa * bk;
@@ -385,12 +449,14 @@ __global__ void __launch_bounds__(256, 4) k_cg_coop(int n, const int* __restrict
         a1 += rk * rk;
         a2 += bk * bk;
     }
-    block_sum2(a0, a1, &pc[3 * blk], &pc[3 * blk + 1]);
-    block_sum2(a2, 0.0, &pc[3 * blk + 2], &pa[2 * blk + 1]);
+    group_sum2(sm, a0, a1, in ? &pc[3 * grp] : nullptr, &pc[3 * grp + 1]);
+    group_sum2(sm, a2, 0.0, in ? &pc[3 * grp + 2] : nullptr, &pa[2 * grp + 1]);
     grid.sync();
-    double rz = grid_total(pc, 3, 0, nb);
-    const double rr0 = grid_total(pc, 3, 1, nb);
-    const double bnorm = sqrt(grid_total(pc, 3, 2, nb));
+    double t3[3], t2[2], t1[1];
+    grid_totals<3>(sm, pc, 3, 0, ng, t3);
+    double rz = t3[0];
+    const double rr0 = t3[1];
+    const double bnorm = sqrt(t3[2]);
     double relres = bnorm > 0.0 ? sqrt(rr0) / bnorm : 0.0;
     int it = 0;
     double beta = 0.0;
@@ -400,30 +466,30 @@ __global__ void __launch_bounds__(256, 4) k_cg_coop(int n, const int* __restrict
         // p' = z + beta p (it > 0), its product and p'.Sp'
         double acc = 0.0;
         for (int k = gtid; k < n; k += gsz) {
-            const double pk = it ? z[k] + beta * pcur[k] : pcur[k];
+            const double qk = pcur[k], zk = z[k], ck = coef[k], fa = farea[k];
+            const int deg = fix[k] ? 0 : nnb[k];
+            const double pk = it ? zk + beta * qk : qk;
             double y = 0.0;
             if (!fix[k]) {
-                const int deg = nnb[k];
-                y = coef[k] * pk;
+                y = ck * pk;
+                for (int s0 = 0; s0 < deg; s0 += CG_SLOTS) {
+                    double o[CG_SLOTS], zj[CG_SLOTS], qj[CG_SLOTS];
+                    int j[CG_SLOTS];
+                    cg_slots(n, k, s0, deg, coef, nbr, o, j);
 #pragma unroll
-                for (int s = 0; s < MAXW; s++) {
-                    if (s < deg) {
-                        const double o = coef[(size_t)(s + 1) * n + k];
-                        const int j = nbr[(size_t)s * n + k];
-                        if (o != 0.0 && j >= 0) {
-                            // the fixed flag and the values are loaded together
-                            // (not the values after the flag): one round trip
-                            const bool fj = fix[j] != 0;
-                            const double zj = it ? z[j] : 0.0;
-                            const double qj = pcur[j];
-                            if (!fj) {
-                                const double pj = it ? zj + beta * qj : qj;
-                                y = y + o * pj;
-                            }
-                        }
+                    for (int t = 0; t < CG_SLOTS; t++) {
+                        zj[t] = z[j[t]];
+                        qj[t] = pcur[j[t]];
                     }
+                    // a fixed neighbour's z and p are zero: it adds nothing
+#pragma unroll
+                    for (int t = 0; t < CG_SLOTS; t++)
+                        if (o[t] != 0.0) {
+                            const double pj = it ? zj[t] + beta * qj[t] : qj[t];
+                            y = y + o[t] * pj;
+                        }
                 }
-                y = farea[k] * y;
+                y = fa * y;
             }
             if (it) pnew[k] = pk;
             ap[k] = y;
@@ -434,32 +500,34 @@ __global__ void __launch_bounds__(256, 4) k_cg_coop(int n, const int* __restrict
             pcur = pnew;
             pnew = t;
         }
-        block_sum2(acc, 0.0, &pa[2 * blk], &pa[2 * blk + 1]);
+        group_sum2(sm, acc, 0.0, in ? &pa[2 * grp] : nullptr, &pa[2 * grp + 1]);
         grid.sync();
-        const double pap = grid_total(pa, 2, 0, nb);
+        grid_totals<1>(sm, pa, 2, 0, ng, t1);
+        const double pap = t1[0];
         const double alpha = (pap != 0.0) ? rz / pap : 0.0;
         double c0 = 0.0, c1 = 0.0;
         for (int k = gtid; k < n; k += gsz) {
+            const double xk = x[k], qk = pcur[k], ok = r[k], yk = ap[k], fa = farea[k], ck = coef[k];
             if (fix[k]) continue;
-            x[k] = x[k] + alpha * pcur[k];
-            const double rk = r[k] - alpha * ap[k];
+            x[k] = xk + alpha * qk;
+            const double rk = ok - alpha * yk;
             r[k] = rk;
-            const double zk = rk / (farea[k] * coef[k]);
+            const double zk = rk / (fa * ck);
             z[k] = zk;
             c0 += rk * zk;
             c1 += rk * rk;
         }
-        block_sum2(c0, c1, &pb[2 * blk], &pb[2 * blk + 1]);
+        group_sum2(sm, c0, c1, in ? &pb[2 * grp] : nullptr, &pb[2 * grp + 1]);
         grid.sync();
-        const double rzn = grid_total(pb, 2, 0, nb);
-        const double rr = grid_total(pb, 2, 1, nb);
+        grid_totals<2>(sm, pb, 2, 0, ng, t2);
+        const double rzn = t2[0], rr = t2[1];
         beta = (rz != 0.0) ? rzn / rz : 0.0;
         rz = rzn;
         relres = sqrt(rr) / bnorm;
         it++;
         if (!(relres == relres) || relres <= rtol || it >= max_iter) break;
     }
-    if (gtid == 0) {
+    if (one) {
         *it_out = it;
         *res_out = relres;
     }
@@ -468,17 +536,21 @@ __global__ void __launch_bounds__(256, 4) k_cg_coop(int n, const int* __restrict
 // FP32 CG (precision form): S d = rhs from d = 0 with FP32 vectors and FP32
 // arithmetic (coefficients rounded on load), dot products accumulated in FP64;
 // the same barrier structure as k_cg_coop.
-__global__ void __launch_bounds__(256) k_cg_coop32(int n, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
+__global__ void __launch_bounds__(CG_GROUP * CG_GROUPS, 1) k_cg_coop32(int n, int ng, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
                                                    const double* __restrict__ coef, const double* __restrict__ farea,
                                                    const uint8_t* __restrict__ fix, const double* __restrict__ rhs,
                                                    float* x, float* r, float* z, float* pp, float* ap, double* part,
                                                    double rtol, int max_iter, int* it_out, double* res_out) {
     cg::grid_group grid = cg::this_grid();
-    const int nb = gridDim.x, blk = blockIdx.x;
-    const int gtid = blk * blockDim.x + threadIdx.x, gsz = nb * blockDim.x;
+    __shared__ double sm[CG_SMEM];
+    // group of this thread; a thread past the last group has no rows
+    const int grp = blockIdx.x + (threadIdx.x / CG_GROUP) * gridDim.x;
+    const bool in = grp < ng;
+    const int gtid = in ? grp * CG_GROUP + (threadIdx.x & (CG_GROUP - 1)) : n, gsz = ng * CG_GROUP;
+    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     double* pc = part;
-    double* pa = part + 3 * nb;
-    double* pb = part + 5 * nb;
+    double* pa = part + 3 * ng;
+    double* pb = part + 5 * ng;
     double a0 = 0.0, a1 = 0.0;
     for (int k = gtid; k < n; k += gsz) {
         x[k] = 0.0f;
@@ -494,10 +566,12 @@ __global__ void __launch_bounds__(256) k_cg_coop32(int n, const int* __restrict_
         a0 += (double)rk * (double)zk;
         a1 += (double)rk * (double)rk;
     }
-    block_sum2(a0, a1, &pc[3 * blk], &pc[3 * blk + 1]);
+    group_sum2(sm, a0, a1, in ? &pc[3 * grp] : nullptr, &pc[3 * grp + 1]);
     grid.sync();
-    double rz = grid_total(pc, 3, 0, nb);
-    const double bnorm = sqrt(grid_total(pc, 3, 1, nb));
+    double t2[2], t1[1];
+    grid_totals<2>(sm, pc, 3, 0, ng, t2);
+    double rz = t2[0];
+    const double bnorm = sqrt(t2[1]);
     double relres = bnorm > 0.0 ? 1.0 : 0.0;
     int it = 0;
     while (bnorm > 0.0 && relres > rtol && it < max_iter) {
@@ -518,9 +592,10 @@ __global__ void __launch_bounds__(256) k_cg_coop32(int n, const int* __restrict_
             ap[k] = y;
             acc += (double)pp[k] * (double)y;
         }
-        block_sum2(acc, 0.0, &pa[2 * blk], &pa[2 * blk + 1]);
+        group_sum2(sm, acc, 0.0, in ? &pa[2 * grp] : nullptr, &pa[2 * grp + 1]);
         grid.sync();
-        const double pap = grid_total(pa, 2, 0, nb);
+        grid_totals<1>(sm, pa, 2, 0, ng, t1);
+        const double pap = t1[0];
         const float alpha = (float)((pap != 0.0) ? rz / pap : 0.0);
         double c0 = 0.0, c1 = 0.0;
         for (int k = gtid; k < n; k += gsz) {
@@ -533,10 +608,10 @@ __global__ void __launch_bounds__(256) k_cg_coop32(int n, const int* __restrict_
             c0 += (double)rk * (double)zk;
             c1 += (double)rk * (double)rk;
         }
-        block_sum2(c0, c1, &pb[2 * blk], &pb[2 * blk + 1]);
+        group_sum2(sm, c0, c1, in ? &pb[2 * grp] : nullptr, &pb[2 * grp + 1]);
         grid.sync();
-        const double rzn = grid_total(pb, 2, 0, nb);
-        const double rr = grid_total(pb, 2, 1, nb);
+        grid_totals<2>(sm, pb, 2, 0, ng, t2);
+        const double rzn = t2[0], rr = t2[1];
         const float beta = (float)((rz != 0.0) ? rzn / rz : 0.0);
         rz = rzn;
         relres = sqrt(rr) / bnorm;
@@ -545,7 +620,7 @@ __global__ void __launch_bounds__(256) k_cg_coop32(int n, const int* __restrict_
         for (int k = gtid; k < n; k += gsz) pp[k] = z[k] + beta * pp[k];
         grid.sync();
     }
-    if (gtid == 0) {
+    if (one) {
         *it_out = it;
         *res_out = relres;
     }
@@ -573,10 +648,19 @@ static int cg_second_direction(gs_plan* p) {
     return GS_OK;
 }
 
-static int cg_launch(gs_plan* p, const void* fn, void** args) {
+// thread groups of the CG: the cooperative blocks of the plan
+static int cg_groups(const gs_plan* p) { return std::min(p->coop_blocks, CG_MAXG); }
+
+// ng groups of 256 threads, as many to a block as an SM's share of them
+static int cg_launch(gs_plan* p, const void* fn, int ng, void** args) {
+    const int per = std::min(CG_GROUPS, (ng + p->sm_count - 1) / p->sm_count);
+    if (ng > CG_MAXG) {
+        set_error(GS_EINVAL, "diffusion CG: more thread groups than the staging of their sums holds");
+        return GS_EINVAL;
+    }
     cudaEvent_t stop = nullptr;
     if (p->profiling) prof_begin(p, fn, &stop);
-    GS_CUDA(cudaLaunchCooperativeKernel(fn, p->coop_blocks, 256, args, 0, p->stream));
+    GS_CUDA(cudaLaunchCooperativeKernel(fn, (ng + per - 1) / per, CG_GROUP * per, args, 0, p->stream));
     if (stop) cudaEventRecord(stop, p->stream);
     p->launches++;
     return GS_OK;
@@ -608,11 +692,12 @@ static int hillslope_refine32(gs_plan* p, double tol, int max_iter, int* outer, 
     for (; it < 10 && relres > tol; it++) {
         int nn = n, mi = max_iter;
         double rt = 1.0e-5;
-        void* args[] = {(void*)&nn, (void*)&p->nbr, (void*)&p->nnb, (void*)&p->dcoef, (void*)&p->farea,
+        int ng = cg_groups(p);
+        void* args[] = {(void*)&nn, (void*)&ng, (void*)&p->nbr, (void*)&p->nnb, (void*)&p->dcoef, (void*)&p->farea,
                         (void*)&p->dfix, (void*)&p->cg_r, (void*)&p->f32a, (void*)&p->f32b, (void*)&p->f32c,
                         (void*)&p->f32d, (void*)&p->f32e, (void*)&p->red, (void*)&rt, (void*)&mi, (void*)&it_d,
                         (void*)&res_d};
-        GS_TRY(cg_launch(p, (const void*)k_cg_coop32, args));
+        GS_TRY(cg_launch(p, (const void*)k_cg_coop32, ng, args));
         launch(p, k_add_f32_d, G, B, n, (const float*)p->f32a, p->cg_x);
         launch(p, k_cg_resid, G, B, n, p->W, p->flat, (const int*)p->nbr, (const int8_t*)p->nnb,
                (const double*)p->dcoef, (const double*)p->farea, (const uint8_t*)p->outlet, (const double*)p->cg_b,
@@ -716,15 +801,12 @@ int hillslope(gs_plan* p, double* h, double* cum_ed, double* eb, double sealevel
         int nn = n, mi = max_iter;
         double rt = rtol;
         const double* x0 = hold;
-        void* args[] = {(void*)&nn, (void*)&p->nbr, (void*)&p->nnb, (void*)&p->dcoef, (void*)&p->farea,
+        int ng = cg_groups(p);
+        void* args[] = {(void*)&nn, (void*)&ng, (void*)&p->nbr, (void*)&p->nnb, (void*)&p->dcoef, (void*)&p->farea,
                         (void*)&p->dfix, (void*)&x0, (void*)&p->cg_x, (void*)&p->cg_b, (void*)&p->cg_r,
                         (void*)&p->cg_z, (void*)&p->cg_p, (void*)&p->cg_p2, (void*)&p->cg_ap, (void*)&p->red,
                         (void*)&rt, (void*)&mi, (void*)&it_d, (void*)&res_d, (void*)&guess};
-        cudaEvent_t stop = nullptr;
-        if (p->profiling) prof_begin(p, (const void*)k_cg_coop, &stop);
-        GS_CUDA(cudaLaunchCooperativeKernel((const void*)k_cg_coop, p->coop_blocks, 256, args, 0, p->stream));
-        if (stop) cudaEventRecord(stop, p->stream);
-        p->launches++;
+        GS_TRY(cg_launch(p, (const void*)k_cg_coop, ng, args));
     }
     launch(p, k_hill_apply, G, B, n, (const double*)hold, (const double*)p->cg_x, dt, h, cum_ed, eb,
            p->hill_dprev);
@@ -777,18 +859,14 @@ int diffusion_solve_on(gs_plan* p, int m, const int* nbr, const int8_t* nnb, con
         int nn = n, mi = max_iter;
         double rt = rtol;
         const double* cf = coef;
-        void* args[] = {(void*)&nn, (void*)&nbr, (void*)&nnb, (void*)&cf, (void*)&farea,
+        // a small sub-mesh (a few lakes) takes about four rows per thread and
+        // no fewer groups than SMs: fewer partials to add at each barrier
+        int ng = std::min(cg_groups(p), std::max(p->sm_count, (n + 4 * B - 1) / (4 * B)));
+        void* args[] = {(void*)&nn, (void*)&ng, (void*)&nbr, (void*)&nnb, (void*)&cf, (void*)&farea,
                         (void*)&fix, (void*)&rhs, (void*)&p->cg_x, (void*)&p->cg_b, (void*)&p->cg_r,
                         (void*)&p->cg_z, (void*)&p->cg_p, (void*)&p->cg_p2, (void*)&p->cg_ap, (void*)&p->red,
                         (void*)&rt, (void*)&mi, (void*)&it_d, (void*)&res_d, (void*)&guess};
-        // a small sub-mesh (a few lakes) takes about four rows per thread and
-        // no fewer blocks than SMs: fewer blocks meet at each grid barrier
-        const int nb = std::min(p->coop_blocks, std::max(p->sm_count, (n + 4 * B - 1) / (4 * B)));
-        cudaEvent_t stop = nullptr;
-        if (p->profiling) prof_begin(p, (const void*)k_cg_coop, &stop);
-        GS_CUDA(cudaLaunchCooperativeKernel((const void*)k_cg_coop, nb, 256, args, 0, p->stream));
-        if (stop) cudaEventRecord(stop, p->stream);
-        p->launches++;
+        GS_TRY(cg_launch(p, (const void*)k_cg_coop, ng, args));
     }
     launch(p, k_copy_d2, G, B, n, (const double*)p->cg_x, x);
     GS_LAUNCH();

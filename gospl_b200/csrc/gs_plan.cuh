@@ -397,12 +397,12 @@ int output_fields(gs_plan* p, const double* h, const double* cum_ed, const doubl
 
 void prof_begin(gs_plan* p, const void* fn, cudaEvent_t* stop);
 int coop_occupancy(int* per_sm);
-__global__ void k_cg_coop32(int n, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
+__global__ void k_cg_coop32(int n, int ng, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
                             const double* __restrict__ coef, const double* __restrict__ farea,
                             const uint8_t* __restrict__ fix, const double* __restrict__ rhs, float* x, float* r,
                             float* z, float* pp, float* ap, double* part, double rtol, int max_iter, int* it_out,
                             double* res_out);
-__global__ void k_cg_coop(int n, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
+__global__ void k_cg_coop(int n, int ng, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
                           const double* __restrict__ coef, const double* __restrict__ farea,
                           const uint8_t* __restrict__ fix, const double* __restrict__ x0, double* x, double* b,
                           double* r, double* z, double* p0, double* p1, double* ap, double* part, double rtol,
