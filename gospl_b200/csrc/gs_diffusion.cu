@@ -372,83 +372,68 @@ __device__ __forceinline__ void cg_slots(int n, int k, int s0, int deg, const do
         }
 }
 
-// Jacobi-PCG on the area-weighted symmetric form S = A (I + L) of the
-// hillslope system, in one cooperative launch:
-//   start x = x0; free rows b = A_k (x0_k - sum over fixed columns o x0_j),
-//   r = b - S x (free columns), z = r / (A_k c_k), p = z;
-//   per iteration  Sp and p.Sp  | grid barrier |  x += a p, r -= a Sp,
-//   z = r / diag, r.z and r.r  | grid barrier |,
-// and the direction update p' = z + b p of the next iteration is made inside
-// its product: each thread forms p'_j = z_j + b p_j of the neighbours it
-// gathers (the same operations as a separate update pass, so the same bits)
-// and writes its own p'_k to the other buffer.  Two barriers per iteration;
-// group partial sums are added in group order by every block.  Fixed rows
-// (flat outlets, no area) keep x = x0.  The gathers of a row issue together in
-// batches of CG_SLOTS (with a branch on each slot they waited for one another).
-__global__ void __launch_bounds__(CG_GROUP * CG_GROUPS, 1) k_cg_coop(int n, int ng, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
-                                                    const double* __restrict__ coef, const double* __restrict__ farea,
-                                                    const uint8_t* __restrict__ fix, const double* __restrict__ x0,
-                                                    double* x, double* b, double* r, double* z, double* p0, double* p1,
-                                                    double* ap, double* part, double rtol, int max_iter, int* it_out,
-                                                    double* res_out, const double* __restrict__ guess) {
-    cg::grid_group grid = cg::this_grid();
-    __shared__ double sm[CG_SMEM];
-    // group of this thread; a thread past the last group has no rows
-    const int grp = blockIdx.x + (threadIdx.x / CG_GROUP) * gridDim.x;
-    const bool in = grp < ng;
-    const int gtid = in ? grp * CG_GROUP + (threadIdx.x & (CG_GROUP - 1)) : n, gsz = ng * CG_GROUP;
-    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
+// start of row k of a solve (b, r, z, p from x0 or the guess) and its terms of
+// the first dots
+__device__ __forceinline__ void cg_start_row(int n, int k, const int* nbr, const int8_t* nnb, const double* coef,
+                                             const double* farea, const uint8_t* fix, const double* x0,
+                                             const double* guess, double* x, double* b, double* r, double* z,
+                                             double* p0, double& a0, double& a1, double& a2) {
+    const double x0k = x0[k];
+    if (fix[k]) {
+        x[k] = x0k;
+        b[k] = 0.0;
+        r[k] = 0.0;
+        z[k] = 0.0;
+        p0[k] = 0.0;
+        return;
+    }
+    // the start: x0 (the right-hand side), or the guess on free rows
+    const double xk = guess ? guess[k] : x0k;
+    x[k] = xk;
+    const int deg = nnb[k];
+    const double ck = coef[k];
+    double bk = x0k;
+    double y = ck * xk;
+    for (int s0 = 0; s0 < deg; s0 += CG_SLOTS) {
+        double o[CG_SLOTS], xj[CG_SLOTS], gj[CG_SLOTS];
+        int j[CG_SLOTS];
+        uint8_t fj[CG_SLOTS];
+        cg_slots(n, k, s0, deg, coef, nbr, o, j);
+#pragma unroll
+        for (int t = 0; t < CG_SLOTS; t++) {
+            xj[t] = x0[j[t]];
+            gj[t] = guess ? guess[j[t]] : xj[t];
+            fj[t] = fix[j[t]];
+        }
+#pragma unroll
+        for (int t = 0; t < CG_SLOTS; t++)
+            if (o[t] != 0.0) {
+                if (fj[t]) bk = bk - o[t] * xj[t];
+                else y = y + o[t] * gj[t];
+            }
+    }
+    const double fa = farea[k];
+    bk = fa * bk;
+    b[k] = bk;
+    const double rk = bk - fa * y;
+    r[k] = rk;
+    const double zk = rk / (fa * ck);
+    z[k] = zk;
+    p0[k] = zk;
+    a0 += rk * zk;
+    a1 += rk * rk;
+    a2 += bk * bk;
+}
+
+// the iterations after the start, on the whole grid
+__device__ __forceinline__ void cg_iterate(cg::grid_group& grid, double* sm, int n, int ng, int grp, bool in, int gtid,
+                                           int gsz, const int* nbr, const int8_t* nnb, const double* coef,
+                                           const double* farea, const uint8_t* fix, double* x, double* r, double* z,
+                                           double* p0, double* p1, double* ap, double* part, double rtol,
+                                           int max_iter, double a0, double a1, double a2, int& it, double& relres) {
     double* pc = part;             // initial dots [3 ng]
     double* pa = part + 3 * ng;    // p.Ap [2 ng]
     double* pb = part + 5 * ng;    // r.z, r.r [2 ng]
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int k = gtid; k < n; k += gsz) {
-        const double x0k = x0[k];
-        if (fix[k]) {
-            x[k] = x0k;
-            b[k] = 0.0;
-            r[k] = 0.0;
-            z[k] = 0.0;
-            p0[k] = 0.0;
-            continue;
-        }
-        // the start: x0 (the right-hand side), or the guess on free rows
-        const double xk = guess ? guess[k] : x0k;
-        x[k] = xk;
-        const int deg = nnb[k];
-        const double ck = coef[k];
-        double bk = x0k;
-        double y = ck * xk;
-        for (int s0 = 0; s0 < deg; s0 += CG_SLOTS) {
-            double o[CG_SLOTS], xj[CG_SLOTS], gj[CG_SLOTS];
-            int j[CG_SLOTS];
-            uint8_t fj[CG_SLOTS];
-            cg_slots(n, k, s0, deg, coef, nbr, o, j);
-#pragma unroll
-            for (int t = 0; t < CG_SLOTS; t++) {
-                xj[t] = x0[j[t]];
-                gj[t] = guess ? guess[j[t]] : xj[t];
-                fj[t] = fix[j[t]];
-            }
-#pragma unroll
-            for (int t = 0; t < CG_SLOTS; t++)
-                if (o[t] != 0.0) {
-                    if (fj[t]) bk = bk - o[t] * xj[t];
-                    else y = y + o[t] * gj[t];
-                }
-        }
-        const double fa = farea[k];
-        bk = fa * bk;
-        b[k] = bk;
-        const double rk = bk - fa * y;
-        r[k] = rk;
-        const double zk = rk / (fa * ck);
-        z[k] = zk;
-        p0[k] = zk;
-        a0 += rk * zk;
-        a1 += rk * rk;
-        a2 += bk * bk;
-    }
     group_sum2(sm, a0, a1, in ? &pc[3 * grp] : nullptr, &pc[3 * grp + 1]);
     group_sum2(sm, a2, 0.0, in ? &pc[3 * grp + 2] : nullptr, &pa[2 * grp + 1]);
     grid.sync();
@@ -457,8 +442,8 @@ __global__ void __launch_bounds__(CG_GROUP * CG_GROUPS, 1) k_cg_coop(int n, int 
     double rz = t3[0];
     const double rr0 = t3[1];
     const double bnorm = sqrt(t3[2]);
-    double relres = bnorm > 0.0 ? sqrt(rr0) / bnorm : 0.0;
-    int it = 0;
+    relres = bnorm > 0.0 ? sqrt(rr0) / bnorm : 0.0;
+    it = 0;
     double beta = 0.0;
     double* pcur = p0;     // direction of the previous iteration
     double* pnew = p1;
@@ -527,10 +512,147 @@ __global__ void __launch_bounds__(CG_GROUP * CG_GROUPS, 1) k_cg_coop(int n, int 
         it++;
         if (!(relres == relres) || relres <= rtol || it >= max_iter) break;
     }
+}
+
+// Jacobi-PCG on the area-weighted symmetric form S = A (I + L) of the
+// hillslope system, in one cooperative launch:
+//   start x = x0; free rows b = A_k (x0_k - sum over fixed columns o x0_j),
+//   r = b - S x (free columns), z = r / (A_k c_k), p = z;
+//   per iteration  Sp and p.Sp  | grid barrier |  x += a p, r -= a Sp,
+//   z = r / diag, r.z and r.r  | grid barrier |,
+// and the direction update p' = z + b p of the next iteration is made inside
+// its product: each thread forms p'_j = z_j + b p_j of the neighbours it
+// gathers (the same operations as a separate update pass, so the same bits)
+// and writes its own p'_k to the other buffer.  Two barriers per iteration;
+// group partial sums are added in group order by every block.  Fixed rows
+// (flat outlets, no area) keep x = x0.  The gathers of a row issue together in
+// batches of CG_SLOTS (with a branch on each slot they waited for one another).
+__global__ void __launch_bounds__(CG_GROUP * CG_GROUPS, 1) k_cg_coop(int n, int ng, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
+                                                    const double* __restrict__ coef, const double* __restrict__ farea,
+                                                    const uint8_t* __restrict__ fix, const double* __restrict__ x0,
+                                                    double* x, double* b, double* r, double* z, double* p0, double* p1,
+                                                    double* ap, double* part, double rtol, int max_iter, int* it_out,
+                                                    double* res_out, const double* __restrict__ guess) {
+    cg::grid_group grid = cg::this_grid();
+    __shared__ double sm[CG_SMEM];
+    // group of this thread; a thread past the last group has no rows
+    const int grp = blockIdx.x + (threadIdx.x / CG_GROUP) * gridDim.x;
+    const bool in = grp < ng;
+    const int gtid = in ? grp * CG_GROUP + (threadIdx.x & (CG_GROUP - 1)) : n, gsz = ng * CG_GROUP;
+    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0, relres;
+    int it;
+    for (int k = gtid; k < n; k += gsz)
+        cg_start_row(n, k, nbr, nnb, coef, farea, fix, x0, guess, x, b, r, z, p0, a0, a1, a2);
+    cg_iterate(grid, sm, n, ng, grp, in, gtid, gsz, nbr, nnb, coef, farea, fix, x, r, z, p0, p1, ap, part, rtol,
+               max_iter, a0, a1, a2, it, relres);
     if (one) {
         *it_out = it;
         *res_out = relres;
     }
+}
+
+// diffusivity of the deposit: C_d = minDiff + K (1 - exp(-dexp dh)), dh below
+// 0.1 m counted as 0, for the lake cells (hillslope.py:1046-1051)
+__device__ __forceinline__ double lake_cd(double h, double zb, double K, double dexp, double mind) {
+    double dd = __dsub_rn(h, zb);
+    if (dd < 0.1) dd = 0.0;
+    return __dadd_rn(mind, __dmul_rn(K, __dsub_rn(1.0, exp(__dmul_rn(-dexp, dd)))));
+}
+
+// nsub x npic solves of (I + dts L(C_d(h))) h = h_start over the m cells of a
+// sub-mesh (compact neighbours nbr, areas farea, fixed rows fix), L from
+// jacobiancoeff with Kp = 0 (functions.F90:1423-1467), in one cooperative
+// launch: a thread builds the row that it solves (its coefficients need no
+// barrier), the solve runs on the whole grid, and the new diffusivities are
+// the one thing that a barrier has to order before the next rows.  hcur holds
+// the start surface and gets the result.  Latency bounds it (a few thousand
+// cells over 148 SMs): a solve and its rows took six launches, 45 us where the
+// solve itself is 25 us.
+struct PicardArgs {
+    int m, n, ng, nsub, npic, max_iter;
+    const int* cell;
+    const int* nbr;
+    const int8_t* nnb;
+    const double* farea;
+    const uint8_t* fix;
+    const double* elen;
+    const double* vdist;
+    const double* zb;
+    double K, dts, rtol;
+    double *hcur, *cd, *hs, *coef, *x, *b, *r, *z, *p0, *p1, *ap, *part, *worst;
+};
+
+__global__ void __launch_bounds__(CG_GROUP * CG_GROUPS, 1) k_picard(const __grid_constant__ PicardArgs a) {
+    cg::grid_group grid = cg::this_grid();
+    __shared__ double sm[CG_SMEM];
+    const int m = a.m, n = a.n;
+    const int grp = blockIdx.x + (threadIdx.x / CG_GROUP) * gridDim.x;
+    const bool in = grp < a.ng;
+    const int gtid = in ? grp * CG_GROUP + (threadIdx.x & (CG_GROUP - 1)) : m, gsz = a.ng * CG_GROUP;
+    for (int k = gtid; k < m; k += gsz) {
+        const int i = a.cell[k];
+        const double h = a.hcur[i];
+        a.x[k] = h;
+        a.hs[k] = h;
+        a.cd[k] = lake_cd(h, a.zb[i], a.K, 0.05, 1.0e-4);
+    }
+    grid.sync();
+    double worst = 0.0;
+    for (int sub = 0; sub < a.nsub; sub++)
+        for (int pic = 0; pic < a.npic; pic++) {
+            double a0 = 0.0, a1 = 0.0, a2 = 0.0, relres;
+            int it;
+            for (int k = gtid; k < m; k += gsz) {
+                const int i = a.cell[k];
+                const double ak = a.farea[k], ck = a.cd[k];
+                const int deg = a.nnb[k];
+                double dg = 0.0;
+                if (ak > 0.0)
+                    for (int s0 = 0; s0 < deg; s0 += 3) {
+                        double vd[3], el[3], cn[3];
+                        int j[3];
+#pragma unroll
+                        for (int t = 0; t < 3; t++) {
+                            const bool has = s0 + t < deg;
+                            j[t] = has ? a.nbr[(size_t)(s0 + t) * m + k] : -1;
+                            vd[t] = has ? a.vdist[(size_t)(s0 + t) * n + i] : 0.0;
+                            el[t] = has ? a.elen[(size_t)(s0 + t) * n + i] : 1.0;
+                        }
+#pragma unroll
+                        for (int t = 0; t < 3; t++) cn[t] = a.cd[j[t] >= 0 ? j[t] : k];
+#pragma unroll
+                        for (int t = 0; t < 3; t++) {
+                            if (s0 + t >= deg) continue;
+                            double o = 0.0;
+                            // a face to a cell outside is closed
+                            if (j[t] >= 0 && vd[t] > 0.0 && ck > 0.0 && cn[t] > 0.0) {
+                                const double c = __ddiv_rn(__dmul_rn(0.5, __dadd_rn(ck, cn[t])), ak);
+                                const double v = __ddiv_rn(__dmul_rn(c, vd[t]), el[t]);
+                                dg = __dadd_rn(dg, v);
+                                o = __dmul_rn(a.dts, -v);
+                            }
+                            a.coef[(size_t)(s0 + t + 1) * m + k] = o;
+                        }
+                    }
+                a.coef[k] = __dadd_rn(__dmul_rn(a.dts, dg), 1.0);
+                cg_start_row(m, k, a.nbr, a.nnb, a.coef, a.farea, a.fix, a.hs, nullptr, a.x, a.b, a.r, a.z, a.p0, a0,
+                             a1, a2);
+            }
+            cg_iterate(grid, sm, m, a.ng, grp, in, gtid, gsz, a.nbr, a.nnb, a.coef, a.farea, a.fix, a.x, a.r, a.z,
+                       a.p0, a.p1, a.ap, a.part, a.rtol, a.max_iter, a0, a1, a2, it, relres);
+            if (!(relres == relres) || relres > worst) worst = relres;   // NaN wins
+            const bool last = pic + 1 == a.npic;
+            for (int k = gtid; k < m; k += gsz) {
+                const int i = a.cell[k];
+                const double h = a.x[k];
+                a.cd[k] = lake_cd(h, a.zb[i], a.K, 0.05, 1.0e-4);
+                if (last) a.hs[k] = h;
+            }
+            grid.sync();
+        }
+    for (int k = gtid; k < m; k += gsz) a.hcur[a.cell[k]] = a.x[k];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.worst = worst;
 }
 
 // FP32 CG (precision form): S d = rhs from d = 0 with FP32 vectors and FP32
@@ -650,6 +772,12 @@ static int cg_second_direction(gs_plan* p) {
 
 // thread groups of the CG: the cooperative blocks of the plan
 static int cg_groups(const gs_plan* p) { return std::min(p->coop_blocks, CG_MAXG); }
+
+// a small sub-mesh (a few lakes) takes about four rows per thread and no fewer
+// groups than SMs: fewer partials to add at each barrier
+static int cg_small_groups(const gs_plan* p, int m) {
+    return std::min(cg_groups(p), std::max(p->sm_count, (m + 4 * CG_GROUP - 1) / (4 * CG_GROUP)));
+}
 
 // ng groups of 256 threads, as many to a block as an SM's share of them
 static int cg_launch(gs_plan* p, const void* fn, int ng, void** args) {
@@ -838,15 +966,23 @@ int hillslope(gs_plan* p, double* h, double* cum_ed, double* eb, double sealevel
 // rows without area held fixed as in the hillslope solve; the cooperative CG on
 // the area-weighted symmetric form.  Used by the non-linear lake diffusion of
 // the sediment step.
-// the worst relative residual of a run of solves (NaN wins), for one check at its end
-__global__ void k_cg_fold(const double* __restrict__ res, double* worst) {
-    const double r = *res, w = *worst;
-    if (!(r == r) || r > w) *worst = r;
+// the lagged-diffusivity solves over the m cells `cell` (k_picard), the worst
+// relative residual (NaN wins) in *worst on the device
+int picard_solve(gs_plan* p, int m, const int* cell, const int* nbr, const int8_t* nnb, const double* farea,
+                 const uint8_t* fix, const double* zb, double K, double dts, double* hcur, double* cd, double* hs,
+                 double* coef, double rtol, int max_iter, double* worst) {
+    GS_TRY(cg_second_direction(p));
+    const int ng = cg_small_groups(p, m);
+    PicardArgs a{m, (int)p->n, ng, p->lake_nsub, p->lake_npic, max_iter, cell, nbr, nnb, farea, fix, p->elen,
+                 p->vdist, zb, K, dts, rtol, hcur, cd, hs, coef, p->cg_x, p->cg_b, p->cg_r, p->cg_z, p->cg_p,
+                 p->cg_p2, p->cg_ap, p->red, worst};
+    void* args[] = {(void*)&a};
+    return cg_launch(p, (const void*)k_picard, ng, args);
 }
 
 int diffusion_solve_on(gs_plan* p, int m, const int* nbr, const int8_t* nnb, const double* farea, const uint8_t* fix,
                        int flat, const uint8_t* outlet, const double* coef, const double* rhs, double* x, double rtol,
-                       int max_iter, int* iters, const double* guess, double* worst) {
+                       int max_iter, int* iters, const double* guess) {
     const int n = m;
     if (n == 0) return GS_OK;
     const int B = 256, G = grid_for(n, B);
@@ -859,9 +995,7 @@ int diffusion_solve_on(gs_plan* p, int m, const int* nbr, const int8_t* nnb, con
         int nn = n, mi = max_iter;
         double rt = rtol;
         const double* cf = coef;
-        // a small sub-mesh (a few lakes) takes about four rows per thread and
-        // no fewer groups than SMs: fewer partials to add at each barrier
-        int ng = std::min(cg_groups(p), std::max(p->sm_count, (n + 4 * B - 1) / (4 * B)));
+        int ng = cg_small_groups(p, n);
         void* args[] = {(void*)&nn, (void*)&ng, (void*)&nbr, (void*)&nnb, (void*)&cf, (void*)&farea,
                         (void*)&fix, (void*)&rhs, (void*)&p->cg_x, (void*)&p->cg_b, (void*)&p->cg_r,
                         (void*)&p->cg_z, (void*)&p->cg_p, (void*)&p->cg_p2, (void*)&p->cg_ap, (void*)&p->red,
@@ -870,13 +1004,6 @@ int diffusion_solve_on(gs_plan* p, int m, const int* nbr, const int8_t* nnb, con
     }
     launch(p, k_copy_d2, G, B, n, (const double*)p->cg_x, x);
     GS_LAUNCH();
-    if (worst) {
-        // the caller checks the worst residual of its solves once, at its end
-        launch(p, k_cg_fold, 1, 1, (const double*)res_d, worst);
-        GS_LAUNCH();
-        if (iters) *iters = 0;
-        return GS_OK;
-    }
     int it = 0;
     double relres = 0.0;
     GS_CUDA(cudaMemcpyAsync(&it, it_d, sizeof(int), cudaMemcpyDeviceToHost, p->stream));

@@ -58,7 +58,7 @@ struct gs_plan {
     double* led_part = nullptr;          // [5][LED_NB] block partial sums of the budget reductions
     double* sed_coef = nullptr;          // [W+1][n] lake diffusion operator (compacted to the lake cells)
     int* lake_i = nullptr;               // [W+1][n]: lake cell list, then the compact neighbour slots
-    double* lake_d = nullptr;            // [3][n]: compact cell areas, right-hand side, solution
+    double* lake_d = nullptr;            // [n]: compact cell areas
     uint8_t* lake_u8 = nullptr;          // [2][n]: compact neighbour counts, fixed rows
     int lake_on = 0;                     // lake deposits of large deep pits by non-linear diffusion (Picard)
     double lake_K = 10.0;                // its diffusivity (nlPitK)
@@ -383,10 +383,13 @@ int sea_change(gs_plan* p, double* h, double* cum_ed, double* eb, const double* 
                const uint8_t* sea, gs_stats* st);
 int picard_diffuse(gs_plan* p, const uint8_t* lmask, const double* zb, double* hcur, double K, double dt,
                    double* cd, double* hstart);
+int picard_solve(gs_plan* p, int m, const int* cell, const int* nbr, const int8_t* nnb, const double* farea,
+                 const uint8_t* fix, const double* zb, double K, double dts, double* hcur, double* cd, double* hs,
+                 double* coef, double rtol, int max_iter, double* worst);
 // guess: start of the free rows (nullptr: the right-hand side)
 int diffusion_solve_on(gs_plan* p, int m, const int* nbr, const int8_t* nnb, const double* farea, const uint8_t* fix,
                        int flat, const uint8_t* outlet, const double* coef, const double* rhs, double* x, double rtol,
-                       int max_iter, int* iters, const double* guess = nullptr, double* worst = nullptr);
+                       int max_iter, int* iters, const double* guess = nullptr);
 int hillslope(gs_plan* p, double* h, double* cum_ed, double* eb, double sealevel, double cda,
               double cdm, double dt, double rtol, int max_iter, gs_stats* st);
 int apply_forces(gs_plan* p, double* h, const double* rain, const double* upsub, double dt,

@@ -386,21 +386,6 @@ __global__ void k_lake_init(int n, const int* __restrict__ pit, const uint8_t* _
     hcur[i] = __dadd_rn(d, zb[i]);
 }
 
-// diffusivity of the deposit: C_d = minDiff + K (1 - exp(-dexp dh)), dh below
-// 0.1 m counted as 0, on the lake cells only (hillslope.py:1046-1051)
-__global__ void k_lake_cd(int n, const uint8_t* __restrict__ lmask, const double* __restrict__ hcur,
-                          const double* __restrict__ zb, double K, double dexp, double mind, double* cd) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double c = 0.0;
-    if (lmask[i]) {
-        double dd = __dsub_rn(hcur[i], zb[i]);
-        if (dd < 0.1) dd = 0.0;
-        c = __dadd_rn(mind, __dmul_rn(K, __dsub_rn(1.0, exp(__dmul_rn(-dexp, dd)))));
-    }
-    cd[i] = c;
-}
-
 // the lake cells as a sub-mesh: faces to other cells carry no diffusivity,
 // so the rows outside are the identity and the solve decouples
 __global__ void k_lake_flag(int n, const uint8_t* __restrict__ lmask, int* flag) {
@@ -427,44 +412,6 @@ __global__ void k_lake_submesh(int m, int n, int W, const int* __restrict__ cell
         const int j = nbr[(size_t)s * n + i];
         nbr_c[(size_t)s * m + li] = (j >= 0 && lmask[j]) ? lid[j] : -1;
     }
-}
-
-// rows of I + dt_sub L(C_d) for the lake cells: jacobiancoeff with Kp = 0
-// (functions.F90:1423-1467), faces closed where either side has no
-// diffusivity
-__global__ void k_lake_rows_c(int m, int n, int W, const int* __restrict__ cell, const int* __restrict__ nbr,
-                              const int8_t* __restrict__ nnb, const double* __restrict__ elen,
-                              const double* __restrict__ vdist, const double* __restrict__ farea,
-                              const double* __restrict__ cd, double dts, const double* __restrict__ hstart,
-                              double* coef_c, double* rhs_c) {
-    int li = blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= m) return;
-    const int k = cell[li];
-    for (int s = 0; s < W; s++) coef_c[(size_t)(s + 1) * m + li] = 0.0;
-    double dg = 0.0;
-    const double ak = farea[k];
-    if (ak > 0.0) {
-        const double ck = cd[k];
-        for (int s = 0; s < nnb[k]; s++) {
-            const double vd = vdist[(size_t)s * n + k];
-            if (!(vd > 0.0)) continue;
-            const int j = nbr[(size_t)s * n + k];
-            const double cn = cd[j];
-            if (ck > 0.0 && cn > 0.0) {
-                const double c = __ddiv_rn(__dmul_rn(0.5, __dadd_rn(ck, cn)), ak);
-                const double v = __ddiv_rn(__dmul_rn(c, vd), elen[(size_t)s * n + k]);
-                dg = __dadd_rn(dg, v);
-                coef_c[(size_t)(s + 1) * m + li] = __dmul_rn(dts, -v);
-            }
-        }
-    }
-    coef_c[li] = __dadd_rn(__dmul_rn(dts, dg), 1.0);
-    rhs_c[li] = hstart[k];
-}
-
-__global__ void k_lake_scatter(int m, const int* __restrict__ cell, const double* __restrict__ x_c, double* hcur) {
-    int li = blockIdx.x * blockDim.x + threadIdx.x;
-    if (li < m) hcur[cell[li]] = x_c[li];
 }
 
 // smoothed deposit (clipped at 0) and its area-weighted volume terms
@@ -630,7 +577,7 @@ int sed_budget(gs_plan* p, double* out16) {
 // other cells closed (_diffuseImplicitPicard, hillslope.py:988-1076, with
 // C_d = 1e-4 + K (1 - exp(-0.05 (h - zb)))): hcur holds the start surface on
 // entry and the result on return; cd and hstart are [n] scratch.  The cells
-// of lmask form a sub-mesh of m rows, each solve is the cooperative CG on it.
+// of lmask form a sub-mesh of m rows, picard_solve runs the solves on it.
 int picard_diffuse(gs_plan* p, const uint8_t* lmask, const double* zb, double* hcur, double K, double dt,
                    double* cd, double* hstart) {
     const int n = (int)p->n;
@@ -640,14 +587,12 @@ int picard_diffuse(gs_plan* p, const uint8_t* lmask, const double* zb, double* h
     if (!p->sed_coef) GS_CUDA(cudaMalloc((void**)&p->sed_coef, sizeof(double) * (size_t)n * (size_t)(W + 1)));
     if (!p->lake_i) {
         GS_CUDA(cudaMalloc((void**)&p->lake_i, sizeof(int) * (size_t)n * (size_t)(W + 1)));
-        GS_CUDA(cudaMalloc((void**)&p->lake_d, sizeof(double) * (size_t)n * 3));
+        GS_CUDA(cudaMalloc((void**)&p->lake_d, sizeof(double) * (size_t)n));
         GS_CUDA(cudaMalloc((void**)&p->lake_u8, (size_t)n * 2));
     }
     int* cell = p->lake_i;
     int* nbr_c = cell + n;
     double* farea_c = p->lake_d;
-    double* rhs_c = farea_c + n;
-    double* x_c = rhs_c + n;
     int8_t* nnb_c = (int8_t*)p->lake_u8;
     uint8_t* fix_c = p->lake_u8 + n;
     launch(p, k_lake_flag, G, B, n, (const uint8_t*)lmask, p->flagbuf);
@@ -670,25 +615,10 @@ int picard_diffuse(gs_plan* p, const uint8_t* lmask, const double* zb, double* h
            farea_c, fix_c);
     GS_LAUNCH();
     const double dts = dt / p->lake_nsub;
-    // the solves' residuals are checked once, after the last one (they feed
-    // only the device): no host round trip between two Picard iterations
+    // the solves' residuals are checked once, after the last one
     double* worst = p->d_scalar + 2;
-    GS_CUDA(cudaMemsetAsync(worst, 0, sizeof(double), p->stream));
-    for (int sub = 0; sub < p->lake_nsub; sub++) {
-        GS_CUDA(cudaMemcpyAsync(hstart, hcur, sizeof(double) * n, cudaMemcpyDeviceToDevice, p->stream));
-        for (int it = 0; it < p->lake_npic; it++) {
-            launch(p, k_lake_cd, G, B, n, (const uint8_t*)lmask, (const double*)hcur, zb, K, 0.05, 1.0e-4,
-                   cd);
-            launch(p, k_lake_rows_c, grid_for(m, B), B, m, n, W, (const int*)cell, (const int*)p->nbr,
-                   (const int8_t*)p->nnb, (const double*)p->elen, (const double*)p->vdist, (const double*)p->farea,
-                   (const double*)cd, dts, (const double*)hstart, p->sed_coef, rhs_c);
-            GS_LAUNCH();
-            GS_TRY(diffusion_solve_on(p, m, nbr_c, nnb_c, farea_c, fix_c, 0, nullptr, p->sed_coef, rhs_c, x_c,
-                                      1.0e-13, 5000, nullptr, nullptr, worst));
-            launch(p, k_lake_scatter, grid_for(m, B), B, m, (const int*)cell, (const double*)x_c, hcur);
-            GS_LAUNCH();
-        }
-    }
+    GS_TRY(picard_solve(p, m, cell, nbr_c, nnb_c, farea_c, fix_c, zb, K, dts, hcur, cd, hstart, p->sed_coef, 1.0e-13,
+                        5000, worst));
     double w = 0.0;
     GS_CUDA(cudaMemcpyAsync(&w, worst, sizeof(double), cudaMemcpyDeviceToHost, p->stream));
     GS_CUDA(cudaStreamSynchronize(p->stream));
