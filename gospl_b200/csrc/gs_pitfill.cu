@@ -49,7 +49,7 @@ __device__ __forceinline__ int agg_append(int* cnt) {
 }
 
 enum { D_MINH = 0, D_LEVEL = 1 };
-enum { I_CHANGED = 0, I_NEXT = 1, I_XRAW = 2, I_XDEDUP = 3, I_NONFINITE = 13 };
+enum { I_CHANGED = 0, I_NEXT = 1, I_BASINS = 2, I_NONFINITE = 13 };
 
 // --------------------------------------------------------------------------
 // reductions
@@ -100,23 +100,48 @@ __global__ void k_classify(int n, const double* __restrict__ h, const double* __
     ledge[c] = e;
 }
 
-__global__ void k_descend(int n, const double* __restrict__ h, const double* __restrict__ dsc,
-                          const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
-                          const int8_t* __restrict__ ledge, int* parent) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    int8_t e = ledge[c];
-    if (e != -1) { parent[c] = c; return; }      // seeds, excluded cells: roots
-    const double level = dsc[D_LEVEL];
-    double bz = h[c] - level;
-    int best = c;
-    for (int s = 0; s < nnb[c]; s++) {
-        int j = nbr[(size_t)s * n + c];
-        if (j < 0 || ledge[j] == -2) continue;
-        double z = h[j] - level;
-        if (z < bz || (z == bz && j < best)) { bz = z; best = j; }
+// The roots get their starting state for k_basin_levels: a seed level -inf and
+// component -1, a local minimum level 0 (below every key; ~0 with `relax`), its
+// own component, no outgoing edge yet (W), no claim, and a place in basin[].
+__global__ void __launch_bounds__(256) k_descend(int n, int relax, const double* __restrict__ h,
+                                                 const double* __restrict__ dsc, const int* __restrict__ nbr,
+                                                 const int8_t* __restrict__ nnb, const int8_t* __restrict__ ledge,
+                                                 int* parent, unsigned long long* L, unsigned long long* W, int* comp,
+                                                 int* claim, int* basin, int* nbasin) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    bool list = false;
+    if (c < n) {
+        const int8_t e = ledge[c];
+        int best = c;
+        if (e == -1) {       // seeds and excluded cells are roots
+            const double level = dsc[D_LEVEL];
+            double bz = h[c] - level;
+            for (int s = 0; s < nnb[c]; s++) {
+                int j = nbr[(size_t)s * n + c];
+                if (j < 0 || ledge[j] == -2) continue;
+                double z = h[j] - level;
+                if (z < bz || (z == bz && j < best)) { bz = z; best = j; }
+            }
+            list = best == c;
+        }
+        parent[c] = best;
+        if (list) {
+            L[c] = relax ? ~0ULL : 0ULL;
+            W[c] = ~0ULL;
+            comp[c] = c;
+            claim[c] = 0;
+        } else if (e >= 0) {
+            L[c] = dkey(-INFINITY);
+            comp[c] = -1;
+        }
     }
-    parent[c] = best;
+    const unsigned full = 0xffffffffu, lists = __ballot_sync(full, list);
+    if (!lists) return;
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(nbasin, __popc(lists));
+    base = __shfl_sync(full, base, 0);
+    if (list) basin[base + __popc(lists & ((1u << lane) - 1u))] = c;
 }
 
 // Pointer jumping towards the basin roots, up to JUMP_HOPS hops per vertex
@@ -140,55 +165,79 @@ __global__ void k_jump(int n, int* parent, int* changed) {
     if (hop == JUMP_HOPS) *changed = 1;
 }
 
-__global__ void k_basin_init(int n, const int* __restrict__ parent, const int8_t* __restrict__ ledge,
-                             unsigned long long* L) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    if (parent[c] == c) L[c] = (ledge[c] >= 0) ? dkey(-INFINITY) : ~0ULL;
-}
-
-__global__ void k_cross_edges(int n, const double* __restrict__ h, const double* __restrict__ dsc,
-                              const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
-                              const int8_t* __restrict__ ledge, const int* __restrict__ root,
-                              int* xu, int* xv, double* xw, int* count, int64_t cap) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    if (ledge[c] == -2) return;
-    const int rc = root[c];
-    // a seed basin keeps level -inf: no edge can lower it
-    if (ledge[rc] >= 0) return;
-    const double level = dsc[D_LEVEL];
-    const double zc = h[c] - level;
-    // one edge per distinct neighbouring basin, with the smallest pass height
-    // (parallel edges of larger weight can never lower a level further)
+// Edges between basins: a cell at a basin's border emits one edge per distinct
+// neighbouring basin, with the key of the smallest pass height (parallel edges
+// of larger weight can never lower a level further), and lowers its basin's
+// lowest outgoing edge W; a seed basin keeps level -inf, so no edge leads to it.
+// Most cells lie inside: they look at their neighbours' roots, all gathers at
+// once, and at no height; a warp reserves its edges at once.
+__global__ void __launch_bounds__(256, 6) k_cross_edges(int n, const double* __restrict__ h,
+                                                        const double* __restrict__ dsc, const int* __restrict__ nbr,
+                                                        const int8_t* __restrict__ nnb,
+                                                        const int8_t* __restrict__ ledge,
+                                                        const int* __restrict__ root, unsigned long long* W, int* xu,
+                                                        int* xv, unsigned long long* xw, int* count, int64_t cap) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int rc = -1, deg = 0;
+    bool border = false;
+    if (c < n && ledge[c] != -2) {
+        rc = root[c];
+        if (ledge[rc] < 0) {
+            deg = nnb[c];
+            for (int s0 = 0; s0 < deg; s0 += 6) {
+                int j[6];
+#pragma unroll
+                for (int t = 0; t < 6; t++) j[t] = s0 + t < deg ? nbr[(size_t)(s0 + t) * n + c] : -1;
+#pragma unroll
+                for (int t = 0; t < 6; t++)
+                    if (j[t] >= 0) border |= root[j[t]] != rc;
+            }
+        }
+    }
+    if (!__any_sync(full, border)) return;
     int rb[MAXW];
     double wb[MAXW];
-    int nb_ = 0;
-    for (int s = 0; s < nnb[c]; s++) {
-        int j = nbr[(size_t)s * n + c];
-        if (j < 0 || ledge[j] == -2) continue;
-        int rj = root[j];
-        if (rj == rc) continue;
-        double zj = h[j] - level;
-        double w = zc > zj ? zc : zj;
-        int q = 0;
-        while (q < nb_ && rb[q] != rj) q++;
-        if (q == nb_) {
-            rb[nb_] = rj;
-            wb[nb_] = w;
-            nb_++;
-        } else if (w < wb[q]) {
-            wb[q] = w;
+    int cnt = 0;
+    if (border) {
+        const double level = dsc[D_LEVEL];
+        const double zc = h[c] - level;
+        unsigned long long low = ~0ULL;
+        for (int s = 0; s < deg; s++) {
+            const int j = nbr[(size_t)s * n + c];
+            if (j < 0) continue;
+            const int rj = root[j];
+            if (rj == rc || ledge[j] == -2) continue;
+            const double zj = h[j] - level;
+            const double w = zc > zj ? zc : zj;
+            low = min(low, dkey(w));
+            int q = 0;
+            while (q < cnt && rb[q] != rj) q++;
+            if (q == cnt) {
+                rb[cnt] = rj;
+                wb[cnt] = w;
+                cnt++;
+            } else if (w < wb[q]) {
+                wb[q] = w;
+            }
         }
+        if (cnt && low < __ldcg(W + rc)) atomicMin(W + rc, low);
     }
-    for (int q = 0; q < nb_; q++) {
-        int pos = agg_append(count);
-        if (pos < cap) {
-            xu[pos] = rc;
-            xv[pos] = rb[q];
-            xw[pos] = wb[q];
+    int incl = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += v;
+    }
+    int base = 0;
+    if (lane == 31 && incl) base = atomicAdd(count, incl);
+    const int64_t pos = (int64_t)__shfl_sync(full, base, 31) + incl - cnt;
+    for (int q = 0; q < cnt; q++)
+        if (pos + q < cap) {
+            xu[pos + q] = rc;
+            xv[pos + q] = rb[q];
+            xw[pos + q] = dkey(wb[q]);
         }
-    }
 }
 
 __global__ void k_fill_final(int n, const double* __restrict__ h, const double* __restrict__ dsc,
@@ -713,66 +762,127 @@ __global__ void __launch_bounds__(BFT_THREADS, 2) k_bfs_tiles(int M, int S, int 
     if (gtid == 0) *rounds_out = rounds;
 }
 
-// Basin-graph edges deduplicated: k_cross_edges emits one edge per boundary
-// cell and neighbouring basin, so a pair of basins is joined by as many
-// parallel edges as it has boundary cells (about twelve per pair on the
-// sphere's relief).  Only the lowest of them can lower a level, so the edges
-// go through an open-addressing table keyed by (u, v) that keeps the smallest
-// weight key, and the relaxation runs over one edge per pair.  The table has
-// a power-of-two size of about four times the pairs of the previous fill;
-// linear probing gives up after XH_PROBES slots, and then the relaxation uses
-// the edges as emitted (*raw = 1) and the next fill gets a larger table.
-__device__ __forceinline__ unsigned long long xh_mix(unsigned long long k) {
-    // the 64-bit finaliser of MurmurHash3 (Appleby)
-    k ^= k >> 33;
-    k *= 0xff51afd7ed558ccdULL;
-    k ^= k >> 33;
-    k *= 0xc4ceb9fe1a85ec53ULL;
-    k ^= k >> 33;
-    return k;
+// Minimax levels of the basin graph by contraction, in one cooperative launch.
+// All paths of a component without a seed leave it over its lowest outgoing
+// edge W or a higher one, and its members reach one another below the height
+// of any edge they leave by, so every member's level is max(level, W), and the
+// component joins the neighbour over one edge of height W (Boruvka's steps); a
+// component that contains a seed (-1) is finished.  One edge, whichever of
+// equal ones claims the component first: over two of them it could join the
+// seed and a neighbour that reaches the seed only higher up.  A round at least
+// halves the components, whatever the length of the chains of basins, and
+// takes two grid barriers:
+//   every basin notes its component, every live edge the components of its
+//   ends (in place: they only coarsen) and lowers W of the first one;
+//   levels are raised to W, and an edge at W joins its components.
+// W is double-buffered, a component clears the other buffer's entry.  It asks
+// for every edge to be listed from both its ends.  Latency bounds it: five or six rounds
+// of 10 to 20 us, 87, 110 and 120 us on a plane of 20,000 and 161,000 vertices
+// and a sphere of 2.6 million.  Relaxing the edges until nothing changes
+// (k_relax_active, after a table of the basin pairs) took 103, 250 and 140 us.
+__device__ __forceinline__ int bg_root(const int* comp, int x) {
+    for (int it = 0; it < 1 << 20; it++) {
+        const int p = ld_relaxed_s32(comp + x);
+        if (p == x || p < 0) return p;
+        x = p;
+    }
+    return x;
 }
 
-constexpr int XH_PROBES = 64;
-
-__global__ void k_xedge_insert(const int* __restrict__ m_count, int cap, const int* __restrict__ xu,
-                               const int* __restrict__ xv, const double* __restrict__ xw,
-                               unsigned long long* hkey, unsigned long long* hval, long long hcap, int* raw) {
-    const int m = *m_count < cap ? *m_count : cap;
+__global__ void __launch_bounds__(1024, 1) k_basin_levels(const int* __restrict__ m_count, int64_t cap,
+                                                         const int* __restrict__ nbasin,
+                                                         const int* __restrict__ basin, int* comp, int* old,
+                                                         int* claim, int* xu,
+                                                         int* xv, const unsigned long long* __restrict__ xw,
+                                                         unsigned long long* W0, unsigned long long* W1,
+                                                         unsigned long long* L, int* flags, int* rounds_out) {
+    cg::grid_group grid = cg::this_grid();
+    const int64_t mc = *m_count;
+    const int m = (int)(mc < cap ? mc : cap), nb = *nbasin;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
-    const unsigned long long mask = (unsigned long long)hcap - 1ULL;
-    for (int e = gtid; e < m; e += gsz) {
-        const unsigned long long key = ((unsigned long long)(unsigned)xu[e] << 32) | (unsigned)xv[e];
-        const unsigned long long w = dkey(xw[e]);
-        unsigned long long s = xh_mix(key) & mask;
-        bool placed = false;
-        for (int probe = 0; probe < XH_PROBES; probe++) {
-            const unsigned long long k = atomicCAS(&hkey[s], ~0ULL, key);
-            if (k == ~0ULL || k == key) {
-                atomicMin(&hval[s], w);
-                placed = true;
-                break;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned long long *W = W0, *Wn = W1;
+    int r = 0;
+    // the first round starts with every basin its own component and W known
+    for (int i = gtid; i < nb; i += gsz) {
+        const int b = basin[i];
+        old[b] = b;
+        W1[b] = ~0ULL;
+    }
+    for (;; r++) {
+        bool live = false;
+        if (r > 0) {
+            for (int i = gtid; i < nb; i += gsz) {
+                const int b = basin[i];
+                const int c = bg_root(comp, b);
+                old[b] = c;
+                if (c != b) asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(comp + b), "r"(c) : "memory");
+                else Wn[b] = ~0ULL;
             }
-            s = (s + 1ULL) & mask;
+            for (int e0 = gtid - lane; e0 < m; e0 += gsz) {
+                const int e = e0 + lane;
+                const int u = e < m ? xu[e] : -1;
+                int cu = -1;
+                unsigned long long w = ~0ULL;
+                if (u >= 0) {
+                    const int v = xv[e];
+                    w = xw[e];
+                    cu = u;
+                    int cv = v;
+                    for (int it = 0; it < 1 << 20; it++) {      // both ends' roots, step by step together
+                        const int pu = ld_relaxed_s32(comp + cu), pv = cv < 0 ? -1 : ld_relaxed_s32(comp + cv);
+                        if (pu == cu && pv == cv) break;
+                        cu = pu;
+                        cv = pv;
+                        if (cu < 0) break;
+                    }
+                    if (cu == cv) cu = -1;
+                    xu[e] = cu;
+                    xv[e] = cv;
+                }
+                live |= cu >= 0;
+                // late rounds have few components: one atomic per warp and component
+                const unsigned same = __match_any_sync(full, cu);
+                const unsigned hi = __reduce_min_sync(same, (unsigned)(w >> 32));
+                const unsigned lo = __reduce_min_sync(same, (unsigned)(w >> 32) == hi ? (unsigned)w : ~0u);
+                if (cu >= 0 && lane == __ffs(same) - 1) {
+                    const unsigned long long low = (unsigned long long)hi << 32 | lo;
+                    if (low < __ldcg(W + cu)) atomicMin(W + cu, low);
+                }
+            }
+            if (__any_sync(0xffffffffu, live) && (threadIdx.x & 31) == 0) flags[r & 1] = 1;
+            grid.sync();
+            if (!*(volatile int*)&flags[r & 1]) break;
         }
-        if (!placed) *raw = 1;
+        if (gtid == 0) flags[(r + 1) & 1] = 0;   // read for the last time before the last barrier but one
+        for (int i = gtid; i < nb; i += gsz) {
+            const int b = basin[i];
+            const int c = old[b];
+            if (c < 0) continue;
+            const unsigned long long w = __ldcg(W + c);
+            if (w != ~0ULL && w > L[b]) L[b] = w;
+        }
+        for (int e = gtid; e < m; e += gsz) {
+            const int u = xu[e];
+            if (u < 0 || xw[e] != __ldcg(W + u) || atomicMax(claim + u, r + 1) == r + 1) continue;
+            const int v = xv[e];
+            for (int it = 0; it < 1 << 20; it++) {
+                int a = bg_root(comp, u), b = v < 0 ? -1 : bg_root(comp, v);
+                if (a == b) break;
+                if (a < b) { const int t = a; a = b; b = t; }
+                if (atomicCAS(comp + a, a, b) == a) break;
+            }
+        }
+        grid.sync();
+        unsigned long long* t = W;
+        W = Wn;
+        Wn = t;
     }
-}
-
-// table -> edge list (any order: the relaxation's fixed point does not depend
-// on it); every used slot is emptied again for the next fill
-__global__ void k_xedge_compact(long long hcap, unsigned long long* hkey, unsigned long long* hval, int* du, int* dv,
-                                unsigned long long* dw, int* count) {
-    const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x, gsz = (long long)gridDim.x * blockDim.x;
-    for (long long s = gtid; s < hcap; s += gsz) {
-        const unsigned long long k = hkey[s];
-        if (k == ~0ULL) continue;
-        const int pos = agg_append(count);
-        du[pos] = (int)(k >> 32);
-        dv[pos] = (int)(unsigned)(k & 0xffffffffULL);
-        dw[pos] = hval[s];
-        hkey[s] = ~0ULL;
-        hval[s] = ~0ULL;
-    }
+    // a basin that no seed is reached from keeps no level
+    for (int i = gtid; i < nb; i += gsz)
+        if (old[basin[i]] >= 0) L[basin[i]] = ~0ULL;
+    if (gtid == 0) *rounds_out = r;
 }
 
 // Minimax relaxation over the basin graph in one cooperative launch:
@@ -787,22 +897,20 @@ __global__ void k_xedge_compact(long long hcap, unsigned long long* hkey, unsign
 // flags: round r sets flags[r % 3], reads it after the barrier and clears
 // flags[(r + 1) % 3]).  Levels only decrease and a round without any change
 // used only final levels, so the result is the fixed point of the all-edges
-// relaxation whatever the order of the updates.
+// relaxation whatever the order of the updates.  For meshes with edges that
+// only one of their ends lists.
 constexpr int RELAX_REG = 2;
 constexpr int RELAX_SUB = 8;
 
-__global__ void __launch_bounds__(256) k_relax_active(const int* __restrict__ m_count, int cap,
-                                                      const int* __restrict__ raw_p, const int* __restrict__ xu,
-                                                      const int* __restrict__ xv, const double* __restrict__ xw,
-                                                      const int* __restrict__ md_count, const int* __restrict__ du,
-                                                      const int* __restrict__ dv,
-                                                      const unsigned long long* __restrict__ dw,
+__global__ void __launch_bounds__(256) k_relax_active(const int* __restrict__ m_count, int64_t cap,
+                                                      const int* __restrict__ xu, const int* __restrict__ xv,
+                                                      const unsigned long long* __restrict__ xw,
                                                       unsigned long long* L, int* flags, int max_rounds,
                                                       int* rounds_out) {
     cg::grid_group grid = cg::this_grid();
-    const bool raw = *raw_p != 0;
-    // raw: the edge count as k_cross_edges left it (its appends stop at the capacity)
-    const int m = raw ? (*m_count < cap ? *m_count : cap) : *md_count;
+    // the edge count as k_cross_edges left it (its appends stop at the capacity)
+    const int64_t mc = *m_count;
+    const int m = (int)(mc < cap ? mc : cap);
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
     int cu[RELAX_REG], cv[RELAX_REG];
     unsigned long long cw[RELAX_REG], last[RELAX_REG];
@@ -814,9 +922,9 @@ __global__ void __launch_bounds__(256) k_relax_active(const int* __restrict__ m_
         cw[q] = 0ULL;
         last[q] = ~0ULL;
         if (e < m) {
-            cu[q] = raw ? xu[e] : du[e];
-            cv[q] = raw ? xv[e] : dv[e];
-            cw[q] = raw ? dkey(xw[e]) : dw[e];
+            cu[q] = xu[e];
+            cv[q] = xv[e];
+            cw[q] = xw[e];
         }
     }
     volatile unsigned long long* VL = L;
@@ -836,12 +944,11 @@ __global__ void __launch_bounds__(256) k_relax_active(const int* __restrict__ m_
             }
         }
         for (int e = gtid + RELAX_REG * gsz; e < m; e += gsz) {
-            const int v = raw ? xv[e] : dv[e];
-            const unsigned long long lv = VL[v];
+            const unsigned long long lv = VL[xv[e]];
             if (lv == ~0ULL) continue;
-            const unsigned long long w = raw ? dkey(xw[e]) : dw[e];
+            const unsigned long long w = xw[e];
             const unsigned long long cand = w > lv ? w : lv;
-            const int u = raw ? xu[e] : du[e];
+            const int u = xu[e];
             if (cand < VL[u] && cand < atomicMin(&L[u], cand)) changed = 1;
         }
         if (__any_sync(0xffffffffu, changed) && (threadIdx.x & 31) == 0) flags[r % 3] = 1;
@@ -1432,10 +1539,10 @@ __global__ void k_pit_masked_fin(int np1, const int* __restrict__ nch, const int
 // --------------------------------------------------------------------------
 // host driver
 // --------------------------------------------------------------------------
-static int launch_coop(gs_plan* p, const void* fn, void** args) {
+static int launch_coop(gs_plan* p, const void* fn, int blocks, int threads, void** args) {
     cudaEvent_t stop = nullptr;
     if (p->profiling) prof_begin(p, fn, &stop);
-    GS_CUDA(cudaLaunchCooperativeKernel(fn, p->coop_blocks, 256, args, 0, p->stream));
+    GS_CUDA(cudaLaunchCooperativeKernel(fn, blocks, threads, args, 0, p->stream));
     if (stop) cudaEventRecord(stop, p->stream);
     p->launches++;
     return GS_OK;
@@ -1733,8 +1840,13 @@ int fill_elevation(gs_plan* p, const double* h, double sealevel, double ofill, d
     // seeds, descent links, roots
     launch(p, k_classify, G, B, n, h, (const double*)p->d_scalar, (const int*)p->nbr,
            (const int8_t*)p->nnb, (const uint8_t*)p->outlet, p->ledge);
-    launch(p, k_descend, G, B, n, h, (const double*)p->d_scalar, (const int*)p->nbr,
-           (const int8_t*)p->nnb, (const int8_t*)p->ledge, p->parent);
+    GS_CUDA(cudaMemsetAsync(p->i_scalar + I_NEXT, 0, sizeof(int) * 2, p->stream));
+    GS_CUDA(cudaMemsetAsync(p->i_scalar + 5, 0, sizeof(int) * 3, p->stream));
+    // W lies in the diffusion's vectors, which no fill runs beside
+    unsigned long long *w0 = (unsigned long long*)p->cg_p, *w1 = (unsigned long long*)p->cg_ap;
+    launch(p, k_descend, G, B, n, p->mutual ? 0 : 1, h, (const double*)p->d_scalar, (const int*)p->nbr,
+           (const int8_t*)p->nnb, (const int8_t*)p->ledge, p->parent, p->basinL, w0, p->comp, p->flagbuf, p->lab,
+           p->i_scalar + I_BASINS);
     GS_LAUNCH();
     for (int round = 0; round < 64; round++) {
         // two launches a round; the flag is cleared between them, so it tells
@@ -1755,45 +1867,30 @@ int fill_elevation(gs_plan* p, const double* h, double sealevel, double ofill, d
         if (round == 63) { set_error(GS_EMAXITER, "pit fill: root search did not converge"); return GS_EMAXITER; }
     }
     // basin graph and minimax levels
-    launch(p, k_basin_init, G, B, n, (const int*)p->parent, (const int8_t*)p->ledge, p->basinL);
-    GS_CUDA(cudaMemsetAsync(p->i_scalar + I_NEXT, 0, sizeof(int), p->stream));
-    launch(p, k_cross_edges, G, B, n, h, (const double*)p->d_scalar, (const int*)p->nbr,
-           (const int8_t*)p->nnb, (const int8_t*)p->ledge, (const int*)p->parent, p->xe_u, p->xe_v,
-           p->xe_w, p->i_scalar + I_NEXT, p->xe_cap);
-    GS_LAUNCH();
     {
-        // the edge count stays on the device: the deduplication and the
-        // relaxation read it, and the host checks it against the capacity at
-        // the next synchronisation
+        // the counts stay on the device: the contraction reads them, and the
+        // host checks the edges against the capacity at the next synchronisation
         const int* mc = p->i_scalar + I_NEXT;
-        int cap = (int)std::min<int64_t>(p->xe_cap, INT_MAX), maxr = 1000000;
-        int* raw = p->i_scalar + I_XRAW;
-        int* mdc = p->i_scalar + I_XDEDUP;
-        GS_CUDA(cudaMemsetAsync(p->i_scalar + I_XRAW, 0, sizeof(int) * 2, p->stream));
-        GS_CUDA(cudaMemsetAsync(p->i_scalar + 5, 0, sizeof(int) * 3, p->stream));
-        if (p->xh_cap > 0) {
-            launch(p, k_xedge_insert, p->sm_count * 8, 256, mc, cap, (const int*)p->xe_u, (const int*)p->xe_v,
-                   (const double*)p->xe_w, p->xh_key, p->xh_val, (long long)p->xh_cap, raw);
-            launch(p, k_xedge_compact, p->sm_count * 8, 256, (long long)p->xh_cap, p->xh_key, p->xh_val, p->xd_u,
-                   p->xd_v, p->xd_w, mdc);
-            GS_LAUNCH();
-        } else {
-            // no table yet (first fill of the plan): the undeduplicated edges
-            launch(p, k_fill_int, 1, 32, 1, raw, 1);
-            GS_LAUNCH();
-        }
+        const int* nbs = p->i_scalar + I_BASINS;
         int* flags = p->i_scalar + 5;
         int* rout = p->i_scalar + I_CHANGED;
-        void* args[] = {(void*)&mc,       (void*)&cap,      (void*)&raw,       (void*)&p->xe_u, (void*)&p->xe_v,
-                        (void*)&p->xe_w,  (void*)&mdc,      (void*)&p->xd_u,   (void*)&p->xd_v, (void*)&p->xd_w,
-                        (void*)&p->basinL, (void*)&flags,   (void*)&maxr,      (void*)&rout};
-        GS_TRY(launch_coop(p, (const void*)k_relax_active, args));
-        // the table's outcome, for its size at the next fill
-        GS_CUDA(cudaMemcpyAsync(p->h_pinned + 11, p->i_scalar + I_XRAW, sizeof(int) * 2, cudaMemcpyDeviceToHost,
-                                p->stream));
-        GS_CUDA(cudaMemcpyAsync(p->h_pinned + 6, p->i_scalar + I_CHANGED, sizeof(int), cudaMemcpyDeviceToHost,
-                                p->stream));
-        GS_CUDA(cudaMemcpyAsync(p->h_pinned + 7, p->i_scalar + I_NEXT, sizeof(int), cudaMemcpyDeviceToHost,
+        int64_t cap = std::min<int64_t>(p->xe_cap, INT_MAX);
+        launch(p, k_cross_edges, G, B, n, h, (const double*)p->d_scalar, (const int*)p->nbr, (const int8_t*)p->nnb,
+               (const int8_t*)p->ledge, (const int*)p->parent, w0, p->xe_u, p->xe_v, p->xe_w, p->i_scalar + I_NEXT,
+               cap);
+        GS_LAUNCH();
+        if (p->mutual) {
+            void* args[] = {(void*)&mc,      (void*)&cap,     (void*)&nbs, (void*)&p->lab, (void*)&p->comp,
+                            (void*)&p->minseed, (void*)&p->flagbuf, (void*)&p->xe_u, (void*)&p->xe_v, (void*)&p->xe_w, (void*)&w0,
+                            (void*)&w1,      (void*)&p->basinL, (void*)&flags, (void*)&rout};
+            GS_TRY(launch_coop(p, (const void*)k_basin_levels, std::min(p->sm_count, grid_for(n, 1024)), 1024, args));
+        } else {
+            int maxr = 1000000;
+            void* args[] = {(void*)&mc,      (void*)&cap,     (void*)&p->xe_u, (void*)&p->xe_v, (void*)&p->xe_w,
+                            (void*)&p->basinL, (void*)&flags, (void*)&maxr,    (void*)&rout};
+            GS_TRY(launch_coop(p, (const void*)k_relax_active, p->coop_blocks, 256, args));
+        }
+        GS_CUDA(cudaMemcpyAsync(p->h_pinned + 6, p->i_scalar + I_CHANGED, sizeof(int) * 2, cudaMemcpyDeviceToHost,
                                 p->stream));
     }
     launch(p, k_fill_final, G, B, n, h, (const double*)p->d_scalar, marine_sl, (const int8_t*)p->ledge,
@@ -1833,34 +1930,6 @@ int fill_elevation(gs_plan* p, const double* h, double sealevel, double ofill, d
     if ((int64_t)p->h_pinned[7] > p->xe_cap) {
         set_error(GS_ENOMEM, "pit fill: cross-edge capacity exceeded");
         return GS_ENOMEM;
-    }
-    // size the deduplication table for the next fill: four times this fill's
-    // basin pairs (its edge count when the pairs are not known: no table yet,
-    // or probing gave up), grown at once, shrunk only when 16 times too large
-    {
-        const bool known = p->xh_cap > 0 && !p->h_pinned[11];
-        const int64_t pairs = known ? (int64_t)p->h_pinned[12] : (int64_t)p->h_pinned[7];
-        const int64_t want = std::max<int64_t>(4 * pairs, 1 << 12);
-        if (want > p->xh_cap || (known && p->xh_cap > 4 * want)) {
-            int64_t cap = 1 << 12;
-            while (cap < want) cap <<= 1;
-            unsigned long long* ptrs[] = {p->xh_key, p->xh_val, p->xd_w};
-            for (unsigned long long* q : ptrs)
-                if (q) cudaFree(q);
-            if (p->xd_u) cudaFree(p->xd_u);
-            if (p->xd_v) cudaFree(p->xd_v);
-            p->xh_key = p->xh_val = p->xd_w = nullptr;
-            p->xd_u = p->xd_v = nullptr;
-            p->xh_cap = 0;
-            GS_CUDA(cudaMalloc((void**)&p->xh_key, sizeof(unsigned long long) * cap));
-            GS_CUDA(cudaMalloc((void**)&p->xh_val, sizeof(unsigned long long) * cap));
-            GS_CUDA(cudaMalloc((void**)&p->xd_u, sizeof(int) * cap));
-            GS_CUDA(cudaMalloc((void**)&p->xd_v, sizeof(int) * cap));
-            GS_CUDA(cudaMalloc((void**)&p->xd_w, sizeof(unsigned long long) * cap));
-            GS_CUDA(cudaMemsetAsync(p->xh_key, 0xff, sizeof(unsigned long long) * cap, p->stream));
-            GS_CUDA(cudaMemsetAsync(p->xh_val, 0xff, sizeof(unsigned long long) * cap, p->stream));
-            p->xh_cap = cap;
-        }
     }
     if (st) st->fill_rounds = p->h_pinned[6];
     const int P = p->npits, np1 = P + 1;

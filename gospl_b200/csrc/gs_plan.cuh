@@ -124,6 +124,7 @@ struct gs_plan {
     double* c = nullptr;                 // SPL coefficients [R][n]
 
     // mesh tiles of the dataflow sweeps (gs_tiles.cu); tl_nt = 0: ordered sweeps
+    bool mutual = true;                  // every edge is listed by both of its ends
     int tl_nt = 0;                       // tiles, one resident block each
     int tl_T = 0;                        // vertices per tile
     int tl_np = 0;                       // predecessor slots of a record (6, 8 or 12)
@@ -149,14 +150,8 @@ struct gs_plan {
     unsigned long long* basinL = nullptr;
     int* xe_u = nullptr;                 // cross edges (basin_u, basin_v, w)
     int* xe_v = nullptr;
-    double* xe_w = nullptr;
+    unsigned long long* xe_w = nullptr;
     int64_t xe_cap = 0;
-    unsigned long long* xh_key = nullptr; // [xh_cap] basin-pair table of the edge deduplication (~0: empty)
-    unsigned long long* xh_val = nullptr; // [xh_cap] smallest weight key of the pair
-    int64_t xh_cap = 0;                   // power of two (0: no table, edges used as emitted)
-    int* xd_u = nullptr;                  // [xh_cap] deduplicated edges
-    int* xd_v = nullptr;
-    unsigned long long* xd_w = nullptr;
     int* bfs_rows = nullptr;             // packed BFS adjacency rows, stride ((W+4)/4)*4
     int* comp = nullptr;
     int* minseed = nullptr;
