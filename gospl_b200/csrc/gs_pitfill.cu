@@ -48,32 +48,55 @@ __device__ __forceinline__ int agg_append(int* cnt) {
     return g.shfl(base, 0) + (int)g.thread_rank();
 }
 
-enum { D_MINH = 0, D_LEVEL = 1 };
-enum { I_CHANGED = 0, I_NEXT = 1, I_BASINS = 2, I_NONFINITE = 13 };
+// d_scalar: smallest height, fill level, level above which cells are labelled
+enum { D_MINH = 0, D_LEVEL = 1, D_LABEL = 3 };
+// u_scalar: min key, non-finite and block count of k_level; the fill's outcome
+enum { U_LEVEL = 8, U_OUT = 12 };
+// words of the outcome, as the host reads them into h_pinned + 6
+enum { F_ROUNDS = 0, F_EDGES, F_PITS, F_NONFINITE, F_CELLS, F_COUNT };
+enum { I_ROUNDS = 0, I_NEXT = 1, I_BASINS = 2, I_FLAGS = 5, I_NONFINITE = 13 };
 
 // --------------------------------------------------------------------------
 // reductions
 // --------------------------------------------------------------------------
-__global__ void k_min_key(int n, const double* __restrict__ x, unsigned long long* out) {
+// Smallest height, fill level, and whether every input is finite, in one pass;
+// the last block to finish (word[2] counts them, from -1) sets the scalars and
+// clears the counters of the kernels that follow.  word[0] and word[1] start as
+// all ones: the smallest key, and 0 once a value is not finite.
+__global__ void __launch_bounds__(256) k_level(int n, const double* __restrict__ x, const double* __restrict__ b,
+                                               unsigned long long* word, int sphere, double sealevel, double ofill,
+                                               int sed, double* dsc, int* isc) {
     unsigned long long best = ~0ULL;
+    bool bad = false;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        unsigned long long k = dkey(x[i]);
+        const double v = x[i];
+        const unsigned long long k = dkey(v);
         best = k < best ? k : best;
+        bad |= !isfinite(v) || (b && !isfinite(b[i]));
     }
     for (int o = 16; o > 0; o >>= 1) {
         unsigned long long v = __shfl_xor_sync(0xffffffffu, best, o);
         best = v < best ? v : best;
     }
-    if ((threadIdx.x & 31) == 0) atomicMin(out, best);
-}
-
-__global__ void k_level(const unsigned long long* minkey, int sphere, double sealevel, double ofill,
-                        double* dsc) {
-    double minh = dkey_inv(*minkey);
+    bad = __any_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(word, best);
+        if (bad) atomicExch(word + 1, 0ULL);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x != 0 || atomicAdd(word + 2, 1ULL) + 2ULL != (unsigned long long)gridDim.x) return;
+    __threadfence();
+    double minh = dkey_inv(__ldcg(word));
     if (sphere) minh += 1.0e-3;
-    double b = sealevel + ofill;
+    const double base = sealevel + ofill;
+    const double level = (base > minh) ? base : minh;   // Python max(minh, base)
     dsc[D_MINH] = minh;
-    dsc[D_LEVEL] = (b > minh) ? b : minh;   // Python max(minh, b)
+    dsc[D_LEVEL] = level;
+    dsc[D_LABEL] = sed ? level : sealevel;
+    isc[I_NONFINITE] = __ldcg(word + 1) == 0ULL ? 1 : 0;
+    isc[I_NEXT] = isc[I_BASINS] = 0;
+    for (int k = 0; k < 3; k++) isc[I_FLAGS + k] = 0;
 }
 
 // --------------------------------------------------------------------------
@@ -103,27 +126,47 @@ __global__ void k_classify(int n, const double* __restrict__ h, const double* __
 // The roots get their starting state for k_basin_levels: a seed level -inf and
 // component -1, a local minimum level 0 (below every key; ~0 with `relax`), its
 // own component, no outgoing edge yet (W), no claim, and a place in basin[].
+// A cell at or above the level next to an excluded one would make it a seed
+// when edges have both ends listed: then no neighbour needs a look at its class,
+// and the cell's own class is found here (CLASS).
+template <bool CLASS>
 __global__ void __launch_bounds__(256) k_descend(int n, int relax, const double* __restrict__ h,
                                                  const double* __restrict__ dsc, const int* __restrict__ nbr,
-                                                 const int8_t* __restrict__ nnb, const int8_t* __restrict__ ledge,
-                                                 int* parent, unsigned long long* L, unsigned long long* W, int* comp,
-                                                 int* claim, int* basin, int* nbasin) {
+                                                 const int8_t* __restrict__ nnb, const uint8_t* __restrict__ outlet,
+                                                 int8_t* ledge, int* parent, unsigned long long* L,
+                                                 unsigned long long* W, int* comp, int* claim, int* basin,
+                                                 int* nbasin) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     bool list = false;
     if (c < n) {
-        const int8_t e = ledge[c];
+        const double level = dsc[D_LEVEL];
+        const double hc = h[c] - level;
+        int8_t e = CLASS ? -1 : ledge[c];
         int best = c;
-        if (e == -1) {       // seeds and excluded cells are roots
-            const double level = dsc[D_LEVEL];
-            double bz = h[c] - level;
-            for (int s = 0; s < nnb[c]; s++) {
-                int j = nbr[(size_t)s * n + c];
-                if (j < 0 || ledge[j] == -2) continue;
-                double z = h[j] - level;
-                if (z < bz || (z == bz && j < best)) { bz = z; best = j; }
+        if (CLASS && outlet[c]) e = 2;
+        if (CLASS ? (e == -1 || hc < 0.0) : e == -1) {       // seeds and excluded cells are roots
+            const int deg = nnb[c];
+            double bz = hc;
+            bool ge = false;
+            for (int s0 = 0; s0 < deg; s0 += 6) {
+                int j[6];
+                double z[6];
+#pragma unroll
+                for (int t = 0; t < 6; t++) j[t] = s0 + t < deg ? nbr[(size_t)(s0 + t) * n + c] : -1;
+#pragma unroll
+                for (int t = 0; t < 6; t++) z[t] = j[t] >= 0 ? h[j[t]] - level : 0.0;
+#pragma unroll
+                for (int t = 0; t < 6; t++) {
+                    if (j[t] < 0 || (!CLASS && ledge[j[t]] == -2)) continue;
+                    ge |= z[t] >= 0.0;
+                    if (z[t] < bz || (z[t] == bz && j[t] < best)) { bz = z[t]; best = j[t]; }
+                }
             }
-            list = best == c;
+            if (CLASS && hc < 0.0) e = ge ? (outlet[c] ? 2 : 0) : -2;
+            if (e != -1) best = c;
+            list = e == -1 && best == c;
         }
+        if (CLASS) ledge[c] = e;
         parent[c] = best;
         if (list) {
             L[c] = relax ? ~0ULL : 0ULL;
@@ -144,25 +187,23 @@ __global__ void __launch_bounds__(256) k_descend(int n, int relax, const double*
     if (list) basin[base + __popc(lists & ((1u << lane) - 1u))] = c;
 }
 
-// Pointer jumping towards the basin roots, up to JUMP_HOPS hops per vertex
-// and launch.  Other threads shorten the same chains concurrently; every
-// parent value ever stored is an ancestor on the vertex's descent path, so
-// reading a stale or a fresh value are both valid steps.  *changed is set
-// while some vertex has not reached its root.
+// Every vertex walks to its basin's root and leaves what it has reached in its
+// own parent on the way.  Other threads shorten the same chains concurrently;
+// every parent value ever stored is an ancestor on the vertex's descent path,
+// so reading a stale or a fresh value are both valid steps, and a path ends: it
+// descends strictly (height, then id).
 constexpr int JUMP_HOPS = 16;
-__global__ void k_jump(int n, int* parent, int* changed) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_jump(int n, int* parent) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n) return;
-    const int p0 = parent[c];
-    int p = p0;
-    int hop = 0;
-    for (; hop < JUMP_HOPS; hop++) {
-        int pp = ld_relaxed_s32(parent + p);
+    int p = parent[c], written = p;
+    for (int hop = 1;; hop++) {
+        const int pp = ld_relaxed_s32(parent + p);
         if (pp == p) break;
         p = pp;
+        if (hop % JUMP_HOPS == 0) parent[c] = written = p;
     }
-    if (p != p0) parent[c] = p;
-    if (hop == JUMP_HOPS) *changed = 1;
+    if (p != written) parent[c] = p;
 }
 
 // Edges between basins: a cell at a basin's border emits one edge per distinct
@@ -240,12 +281,26 @@ __global__ void __launch_bounds__(256, 6) k_cross_edges(int n, const double* __r
         }
 }
 
+// The filled surface, and the starting values of the labels and pit tables.
+// An input that is not finite leaves lfill as it was.
 __global__ void k_fill_final(int n, const double* __restrict__ h, const double* __restrict__ dsc,
                              double sealevel, const int8_t* __restrict__ ledge,
                              const int* __restrict__ root, const unsigned long long* __restrict__ L,
-                             double* lfill) {
+                             const int* __restrict__ isc, double* lfill, int* minseed, int* present, int* bestlid,
+                             int* spill_flag, int* seg_count) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n) return;
+    minseed[c] = INT_MAX;
+    present[c] = 0;
+    bestlid[c] = INT_MAX;
+    spill_flag[c] = 0;
+    seg_count[c] = 0;
+    if (c == 0) {
+        present[n] = 0;
+        bestlid[n] = INT_MAX;
+        seg_count[n] = seg_count[n + 1] = 0;
+    }
+    if (isc[I_NONFINITE]) return;
     const double level = dsc[D_LEVEL];
     const double hs = h[c] - level;
     double f = hs;
@@ -275,16 +330,12 @@ __device__ int uf_root(int* comp, int x) {
     return x;
 }
 
-__global__ void k_fill_int(int n, int* a, int v) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = v;
-}
-
 // union-find start: every cell above sea level points to its smallest-id
 // equal-fill neighbour (or itself), so the linking pass starts from short
 // chains instead of singletons
-__global__ void k_uf_init(int n, const double* __restrict__ f, double sl, const int* __restrict__ nbr,
+__global__ void k_uf_init(int n, const double* __restrict__ f, const double* __restrict__ dsc, const int* __restrict__ nbr,
                           const int8_t* __restrict__ nnb, int* comp) {
+    const double sl = dsc[D_LABEL];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int best = i;
@@ -298,8 +349,9 @@ __global__ void k_uf_init(int n, const double* __restrict__ f, double sl, const 
     comp[i] = best;
 }
 
-__global__ void k_uf_link(int n, const double* __restrict__ f, double sl, const int* __restrict__ nbr,
+__global__ void k_uf_link(int n, const double* __restrict__ f, const double* __restrict__ dsc, const int* __restrict__ nbr,
                           const int8_t* __restrict__ nnb, int* comp) {
+    const double sl = dsc[D_LABEL];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double fi = f[i];
@@ -316,35 +368,35 @@ __global__ void k_uf_link(int n, const double* __restrict__ f, double sl, const 
     }
 }
 
-__global__ void k_uf_flatten(int n, int* comp) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) comp[i] = uf_root(comp, i);
-}
 
-__global__ void k_minseed(int n, const double* __restrict__ f, double sl, const int* __restrict__ nbr,
-                          const int8_t* __restrict__ nnb, const int* __restrict__ comp, int* minseed) {
+__global__ void k_minseed(int n, const double* __restrict__ f, const double* __restrict__ dsc,
+                          const int* __restrict__ nbr, const int8_t* __restrict__ nnb, int* comp, int* minseed) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double fi = f[i];
-    if (!(fi > sl)) return;
+    if (!(fi > dsc[D_LABEL])) return;   // alone in its component
+    const int r = uf_root(comp, i);
+    comp[i] = r;
     for (int s = 0; s < nnb[i]; s++) {
         int j = nbr[(size_t)s * n + i];
         if (j >= 0 && fi > f[j]) return;
     }
-    atomicMin(&minseed[comp[i]], i);
+    atomicMin(&minseed[r], i);
 }
 
-__global__ void k_seed_flag(int n, const double* __restrict__ f, double sl, const int* __restrict__ comp,
+__global__ void k_seed_flag(int n, const double* __restrict__ f, const double* __restrict__ dsc, const int* __restrict__ comp,
                             const int* __restrict__ minseed, int* flag) {
+    const double sl = dsc[D_LABEL];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     flag[i] = (f[i] > sl && minseed[comp[i]] == i) ? 1 : 0;
 }
 
 // label (1..P0) per cell, then outlets removed; present[label] marks survivors
-__global__ void k_label(int n, const double* __restrict__ f, double sl, const int* __restrict__ comp,
+__global__ void k_label(int n, const double* __restrict__ f, const double* __restrict__ dsc, const int* __restrict__ comp,
                         const int* __restrict__ minseed, const int* __restrict__ rank,
                         const uint8_t* __restrict__ outlet, int* lab, int* present) {
+    const double sl = dsc[D_LABEL];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int l = -1;
@@ -357,11 +409,36 @@ __global__ void k_label(int n, const double* __restrict__ f, double sl, const in
     if (l > 0) present[l] = 1;
 }
 
-__global__ void k_relabel(int n, const int* __restrict__ lab, const int* __restrict__ newid, int* pit) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int l = lab[i];
-    pit[i] = (l > 0) ? newid[l] + 1 : -1;
+// final pit ids, the sea mask when it is asked for (lFill before the flat pass
+// resets open-sea cells to h: the reset keeps lFill <= sea level), the cells of
+// every pit (one atomic per warp inside a pit), their flags for the compaction,
+// and no flat distance.  An input that is not finite leaves pit and sea alone.
+__global__ void __launch_bounds__(256) k_relabel(int n, const int* __restrict__ lab, const int* __restrict__ newid,
+                                                 const int* __restrict__ isc, const double* __restrict__ f,
+                                                 double sealevel, uint8_t* sea, int* pit, int* flag, int* counts,
+                                                 int* pdir) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned full = 0xffffffffu;
+    const bool ok = isc[I_NONFINITE] == 0;
+    int p = -1;
+    if (i < n) {
+        const int l = lab[i];
+        p = (l > 0) ? newid[l] + 1 : -1;
+        if (ok) {
+            pit[i] = p;
+            if (sea) sea[i] = f[i] <= sealevel ? 1 : 0;
+        }
+        flag[i] = p >= 0 ? 1 : 0;
+        pdir[i] = -1;
+    }
+    const unsigned in = __ballot_sync(full, p >= 0);
+    if (!in) return;
+    const int first = __ffs(in) - 1, p0 = __shfl_sync(full, p, first);
+    if (__all_sync(full, p < 0 || p == p0)) {
+        if ((threadIdx.x & 31) == first) atomicAdd(&counts[p0], __popc(in));
+    } else if (p >= 0) {
+        atomicAdd(&counts[p], 1);
+    }
 }
 
 // --------------------------------------------------------------------------
@@ -398,7 +475,7 @@ __global__ void k_spill_qual(int n, const double* __restrict__ f, const int* __r
 __global__ void k_spill_pick(int np1, int n, const double* __restrict__ f, const int* __restrict__ pit,
                              const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
                              const uint8_t* __restrict__ outlet, const int* __restrict__ bestlid,
-                             int* pit_info, int* spill_flag) {
+                             int* pit_info, int* spill_flag, int* pdir) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np1) return;
     int spill = -1, rank = -1;
@@ -420,6 +497,7 @@ __global__ void k_spill_pick(int np1, int n, const double* __restrict__ f, const
         }
         rank = 0;
         spill_flag[spill] = 1;
+        pdir[spill] = 1;
     }
     pit_info[2 * p] = spill;
     pit_info[2 * p + 1] = rank;
@@ -1265,36 +1343,21 @@ __global__ void k_flat_dirs(int n, const double* __restrict__ f, const int* __re
 // --------------------------------------------------------------------------
 // pit tables
 // --------------------------------------------------------------------------
-// pit cells flagged and counted, and the flat distances' start (1 at spill
-// nodes, else -1).  Neighbouring ids mostly share a depression: its count is
-// one atomic per warp then.
-__global__ void k_pit_flag(int n, const int* __restrict__ pit, const int* __restrict__ spill_flag, int* flag,
-                           int* counts, int* pdir) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned full = 0xffffffffu;
-    int p = -1;
-    if (i < n) {
-        p = pit[i];
-        flag[i] = p >= 0 ? 1 : 0;
-        pdir[i] = spill_flag[i] ? 1 : -1;
-    }
-    const unsigned in = __ballot_sync(full, p >= 0);
-    if (!in) return;
-    const int first = __ffs(in) - 1, p0 = __shfl_sync(full, p, first);
-    if (__all_sync(full, p < 0 || p == p0)) {
-        if ((threadIdx.x & 31) == first) atomicAdd(&counts[p0], __popc(in));
-    } else if (p >= 0) {
-        atomicAdd(&counts[p], 1);
-    }
-}
-
-__global__ void k_pit_compact(int n, const int* __restrict__ pit, const int* __restrict__ pos,
-                              int* keys, int* vals) {
+// pit cells in id order, and the sizes and checks that the host waits for
+__global__ void k_pit_compact(int n, const int* __restrict__ flag, const int* __restrict__ pos,
+                              const int* __restrict__ pit, const int* __restrict__ isc, int* keys, int* vals,
+                              int* out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    int p = pit[i];
-    if (p < 0) return;
-    keys[pos[i]] = p;
+    if (i == n - 1) {
+        out[F_ROUNDS] = isc[I_ROUNDS];
+        out[F_EDGES] = isc[I_NEXT];
+        out[F_PITS] = vals[n] + keys[n];   // labels in use: their scan and flags, not yet overwritten there
+        out[F_NONFINITE] = isc[I_NONFINITE];
+        out[F_CELLS] = pos[i] + flag[i];
+    }
+    if (!flag[i]) return;
+    keys[pos[i]] = pit[i];
     vals[pos[i]] = i;
 }
 
@@ -1591,12 +1654,6 @@ static int bfs_tiles(gs_plan* p, int M, int S, const int* rows, int* ld) {
     return GS_OK;
 }
 
-static int read_ints(gs_plan* p, int* dst, const int* src, int count) {
-    GS_CUDA(cudaMemcpyAsync(dst, src, sizeof(int) * count, cudaMemcpyDeviceToHost, p->stream));
-    GS_CUDA(cudaStreamSynchronize(p->stream));
-    return GS_OK;
-}
-
 static int exclusive_scan(gs_plan* p, const int* in, int* out, int count) {
     size_t bytes = p->cub_bytes;
     GS_CUDA(cub::DeviceScan::ExclusiveSum(p->cub_tmp, bytes, in, out, count, p->stream));
@@ -1792,12 +1849,6 @@ int fill_join(gs_plan* p, gs_stats* st) {
     return GS_OK;
 }
 
-// 1 in *flag when a or b (may be null) holds a NaN or an infinity
-__global__ void k_nonfinite(int n, const double* __restrict__ a, const double* __restrict__ b, int* flag) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (!isfinite(a[i]) || (b && !isfinite(b[i]))) *flag = 1;
-}
 
 int fill_elevation(gs_plan* p, const double* h, double sealevel, double ofill, double* lfill,
                    int* pit_ids, int* flat_dirs, gs_stats* st, bool defer_flats, uint8_t* sea_out, bool sed,
@@ -1809,71 +1860,41 @@ int fill_elevation(gs_plan* p, const double* h, double sealevel, double ofill, d
     }
     if (n == 0) { p->npits = 0; return GS_OK; }
     const int B = 256, G = grid_for(n, B);
-    int hbuf[4];
-    // the inputs must be finite: checked on the device now, read at the
-    // first synchronisation below (the root search), before the relaxation,
-    // the flat pass and any sweep
-    GS_CUDA(cudaMemsetAsync(p->i_scalar + I_NONFINITE, 0, sizeof(int), p->stream));
-    launch(p, k_nonfinite, G, B, n, h, check_b, p->i_scalar + I_NONFINITE);
-    GS_LAUNCH();
-    GS_CUDA(cudaMemcpyAsync(p->h_pinned + 9, p->i_scalar + I_NONFINITE, sizeof(int), cudaMemcpyDeviceToHost,
-                            p->stream));
-
-    // level
-    GS_CUDA(cudaMemsetAsync(p->u_scalar, 0xff, sizeof(unsigned long long), p->stream));
-    launch(p, k_min_key, p->sm_count * 4, 256, n, h, p->u_scalar);
-    launch(p, k_level, 1, 1, (const unsigned long long*)p->u_scalar, p->flat ? 0 : 1, sealevel, ofill,
-           p->d_scalar);
-    GS_LAUNCH();
+    // smallest height, level, and whether the inputs are finite: the host reads
+    // that with the sizes, the kernels until then leave the outputs alone if not
+    // (launches and host waits bound a fill of a small mesh: with a wait for the
+    // check and the roots, one for the pits and one for their cells, and a kernel
+    // or memset per array, a flow accumulation of 20,000 vertices took 790 us, now
+    // 680)
+    unsigned long long* word = p->u_scalar + U_LEVEL;
+    int* out = (int*)(p->u_scalar + U_OUT);
+    GS_CUDA(cudaMemsetAsync(word, 0xff, 3 * sizeof(unsigned long long), p->stream));
+    launch(p, k_level, std::min(p->sm_count * 4, G), 256, n, h, check_b, word, p->flat ? 0 : 1, sealevel, ofill,
+           sed ? 1 : 0, p->d_scalar, p->i_scalar);
     // Filling with sediment (pitfilling.py:557-702, 704-847 with sed=True):
     // open-sea depressions are filled too, pits are labelled above the fill
     // level instead of sea level, and pit volumes use the unclipped surface.
-    double label_sl = sealevel, clip_sl = sealevel, marine_sl = sealevel;
-    if (sed) {
-        GS_CUDA(cudaMemcpyAsync(&label_sl, p->d_scalar + D_LEVEL, sizeof(double), cudaMemcpyDeviceToHost,
-                                p->stream));
-        GS_CUDA(cudaStreamSynchronize(p->stream));
-        clip_sl = -INFINITY;
-        marine_sl = -INFINITY;
-    }
+    const double clip_sl = sed ? -INFINITY : sealevel, marine_sl = sed ? -INFINITY : sealevel;
+    const double* dsc = p->d_scalar;
 
-    // seeds, descent links, roots
-    launch(p, k_classify, G, B, n, h, (const double*)p->d_scalar, (const int*)p->nbr,
-           (const int8_t*)p->nnb, (const uint8_t*)p->outlet, p->ledge);
-    GS_CUDA(cudaMemsetAsync(p->i_scalar + I_NEXT, 0, sizeof(int) * 2, p->stream));
-    GS_CUDA(cudaMemsetAsync(p->i_scalar + 5, 0, sizeof(int) * 3, p->stream));
-    // W lies in the diffusion's vectors, which no fill runs beside
+    // seeds, descent links, roots; W lies in the diffusion's vectors, which no
+    // fill runs beside
     unsigned long long *w0 = (unsigned long long*)p->cg_p, *w1 = (unsigned long long*)p->cg_ap;
-    launch(p, k_descend, G, B, n, p->mutual ? 0 : 1, h, (const double*)p->d_scalar, (const int*)p->nbr,
-           (const int8_t*)p->nnb, (const int8_t*)p->ledge, p->parent, p->basinL, w0, p->comp, p->flagbuf, p->lab,
-           p->i_scalar + I_BASINS);
-    GS_LAUNCH();
-    for (int round = 0; round < 64; round++) {
-        // two launches a round; the flag is cleared between them, so it tells
-        // whether the second one still met a chain longer than JUMP_HOPS (a
-        // launch in which every vertex reached its root leaves the roots)
-        GS_CUDA(cudaMemsetAsync(p->i_scalar + I_CHANGED, 0, sizeof(int), p->stream));
-        launch(p, k_jump, G, B, n, p->parent, p->i_scalar + I_CHANGED);
-        GS_CUDA(cudaMemsetAsync(p->i_scalar + I_CHANGED, 0, sizeof(int), p->stream));
-        launch(p, k_jump, G, B, n, p->parent, p->i_scalar + I_CHANGED);
-        GS_LAUNCH();
-        GS_TRY(read_ints(p, hbuf, p->i_scalar + I_CHANGED, 1));
-        if (round == 0 && p->h_pinned[9]) {
-            set_error(GS_ENONFINITE, check_b ? "non-finite elevation or rain volume (NaN or Inf)"
-                                             : "non-finite elevation (NaN or Inf)");
-            return GS_ENONFINITE;
-        }
-        if (!hbuf[0]) break;
-        if (round == 63) { set_error(GS_EMAXITER, "pit fill: root search did not converge"); return GS_EMAXITER; }
-    }
+    if (!p->mutual)
+        launch(p, k_classify, G, B, n, h, dsc, (const int*)p->nbr, (const int8_t*)p->nnb, (const uint8_t*)p->outlet,
+               p->ledge);
+    launch(p, p->mutual ? k_descend<true> : k_descend<false>, G, B, n, p->mutual ? 0 : 1, h, dsc, (const int*)p->nbr,
+           (const int8_t*)p->nnb, (const uint8_t*)p->outlet, p->ledge, p->parent, p->basinL, w0, p->comp, p->flagbuf,
+           p->lab, p->i_scalar + I_BASINS);
+    launch(p, k_jump, G, B, n, p->parent);
     // basin graph and minimax levels
     {
         // the counts stay on the device: the contraction reads them, and the
-        // host checks the edges against the capacity at the next synchronisation
+        // host checks the edges against the capacity with the sizes
         const int* mc = p->i_scalar + I_NEXT;
         const int* nbs = p->i_scalar + I_BASINS;
-        int* flags = p->i_scalar + 5;
-        int* rout = p->i_scalar + I_CHANGED;
+        int* flags = p->i_scalar + I_FLAGS;
+        int* rout = p->i_scalar + I_ROUNDS;
         int64_t cap = std::min<int64_t>(p->xe_cap, INT_MAX);
         launch(p, k_cross_edges, G, B, n, h, (const double*)p->d_scalar, (const int*)p->nbr, (const int8_t*)p->nnb,
                (const int8_t*)p->ledge, (const int*)p->parent, w0, p->xe_u, p->xe_v, p->xe_w, p->i_scalar + I_NEXT,
@@ -1890,64 +1911,59 @@ int fill_elevation(gs_plan* p, const double* h, double sealevel, double ofill, d
                             (void*)&p->basinL, (void*)&flags, (void*)&maxr,    (void*)&rout};
             GS_TRY(launch_coop(p, (const void*)k_relax_active, p->coop_blocks, 256, args));
         }
-        GS_CUDA(cudaMemcpyAsync(p->h_pinned + 6, p->i_scalar + I_CHANGED, sizeof(int) * 2, cudaMemcpyDeviceToHost,
-                                p->stream));
     }
-    launch(p, k_fill_final, G, B, n, h, (const double*)p->d_scalar, marine_sl, (const int8_t*)p->ledge,
-           (const int*)p->parent, (const unsigned long long*)p->basinL, lfill);
+    launch(p, k_fill_final, G, B, n, h, dsc, marine_sl, (const int8_t*)p->ledge, (const int*)p->parent,
+           (const unsigned long long*)p->basinL, (const int*)p->i_scalar, lfill, p->minseed, p->seg_keys, p->bestlid,
+           p->spill_flag, p->seg_count);
     GS_LAUNCH();
 
-    // label_pits: equal-fill components of cells above sea level
-    launch(p, k_uf_init, G, B, n, (const double*)lfill, label_sl, (const int*)p->nbr, (const int8_t*)p->nnb,
-           p->comp);
-    launch(p, k_uf_link, G, B, n, (const double*)lfill, label_sl, (const int*)p->nbr,
-           (const int8_t*)p->nnb, p->comp);
-    launch(p, k_uf_flatten, G, B, n, p->comp);
-    launch(p, k_fill_int, G, B, n, p->minseed, (int)INT_MAX);
-    GS_LAUNCH();
-    launch(p, k_minseed, G, B, n, (const double*)lfill, label_sl, (const int*)p->nbr,
-           (const int8_t*)p->nnb, (const int*)p->comp, p->minseed);
-    launch(p, k_seed_flag, G, B, n, (const double*)lfill, label_sl, (const int*)p->comp,
-           (const int*)p->minseed, p->flagbuf);
+    // label_pits: equal-fill components of cells above the label level
+    launch(p, k_uf_init, G, B, n, (const double*)lfill, dsc, (const int*)p->nbr, (const int8_t*)p->nnb, p->comp);
+    launch(p, k_uf_link, G, B, n, (const double*)lfill, dsc, (const int*)p->nbr, (const int8_t*)p->nnb, p->comp);
+    launch(p, k_minseed, G, B, n, (const double*)lfill, dsc, (const int*)p->nbr, (const int8_t*)p->nnb, p->comp,
+           p->minseed);
+    launch(p, k_seed_flag, G, B, n, (const double*)lfill, dsc, (const int*)p->comp, (const int*)p->minseed,
+           p->flagbuf);
     GS_LAUNCH();
     GS_TRY(exclusive_scan(p, p->flagbuf, p->scanbuf, n));
-    GS_CUDA(cudaMemsetAsync(p->seg_keys, 0, sizeof(int) * (n + 1), p->stream));  // present[]
-    launch(p, k_label, G, B, n, (const double*)lfill, label_sl, (const int*)p->comp,
-           (const int*)p->minseed, (const int*)p->scanbuf, (const uint8_t*)p->outlet, p->lab,
-           p->seg_keys);
+    launch(p, k_label, G, B, n, (const double*)lfill, dsc, (const int*)p->comp, (const int*)p->minseed,
+           (const int*)p->scanbuf, (const uint8_t*)p->outlet, p->lab, p->seg_keys);
     GS_LAUNCH();
-    // consecutive ids over surviving labels (pits_cons)
+    // consecutive ids over surviving labels (pits_cons); pit cells, compacted in
+    // id order for the flat pass and the per-pit reductions
     GS_TRY(exclusive_scan(p, p->seg_keys, p->seg_vals, n + 1));
-    launch(p, k_relabel, G, B, n, (const int*)p->lab, (const int*)p->seg_vals, pit_ids);
+    launch(p, k_relabel, G, B, n, (const int*)p->lab, (const int*)p->seg_vals, (const int*)p->i_scalar,
+           (const double*)lfill, sealevel, sea_out, pit_ids, p->pflag, p->seg_count, p->pdir);
     GS_LAUNCH();
-    {
-        int last[2];
-        GS_CUDA(cudaMemcpyAsync(&last[0], p->seg_vals + n, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
-        GS_CUDA(cudaMemcpyAsync(&last[1], p->seg_keys + n, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
-        GS_CUDA(cudaStreamSynchronize(p->stream));
-        p->npits = last[0] + last[1];
+    GS_TRY(exclusive_scan(p, p->pflag, p->pscan, n));
+    launch(p, k_pit_compact, G, B, n, (const int*)p->pflag, (const int*)p->pscan, (const int*)pit_ids,
+           (const int*)p->i_scalar, p->seg_keys, p->seg_vals, out);
+    GS_LAUNCH();
+    GS_CUDA(cudaMemcpyAsync(p->h_pinned + 6, out, sizeof(int) * F_COUNT, cudaMemcpyDeviceToHost, p->stream));
+    GS_CUDA(cudaStreamSynchronize(p->stream));
+    const int* res = p->h_pinned + 6;
+    if (res[F_NONFINITE]) {
+        set_error(GS_ENONFINITE, check_b ? "non-finite elevation or rain volume (NaN or Inf)"
+                                         : "non-finite elevation (NaN or Inf)");
+        return GS_ENONFINITE;
     }
-    if ((int64_t)p->h_pinned[7] > p->xe_cap) {
+    p->npits = res[F_PITS];
+    const int ncell = res[F_CELLS];
+    if ((int64_t)res[F_EDGES] > p->xe_cap) {
         set_error(GS_ENOMEM, "pit fill: cross-edge capacity exceeded");
         return GS_ENOMEM;
     }
-    if (st) st->fill_rounds = p->h_pinned[6];
+    if (st) st->fill_rounds = res[F_ROUNDS];
     const int P = p->npits, np1 = P + 1;
     if (st) st->npits = P;
 
     // spill points
-    launch(p, k_fill_int, grid_for(np1, B), B, np1, p->bestlid, (int)INT_MAX);
-    GS_CUDA(cudaMemsetAsync(p->spill_flag, 0, sizeof(int) * n, p->stream));
     launch(p, k_spill_qual, G, B, n, (const double*)lfill, (const int*)pit_ids, (const int*)p->nbr,
            (const int8_t*)p->nnb, (const uint8_t*)p->outlet, p->bestlid);
     launch(p, k_spill_pick, grid_for(np1, B), B, np1, n, (const double*)lfill, (const int*)pit_ids,
            (const int*)p->nbr, (const int8_t*)p->nnb, (const uint8_t*)p->outlet,
-           (const int*)p->bestlid, p->pit_info, p->spill_flag);
+           (const int*)p->bestlid, p->pit_info, p->spill_flag, p->pdir);
     GS_LAUNCH();
-
-    // seaID before the flat pass resets open-sea cells to h (the reset keeps
-    // lFill <= sea level, so the mask is the same before and after it)
-    if (sea_out) GS_TRY(sea_mask(p, lfill, sealevel, sea_out));
 
     // flat distances (fill_dir + nghb_dir fixed point = BFS hop distance).
     // The search and the flat directions run on side_b, beside the pit tables
@@ -1956,23 +1972,13 @@ int fill_elevation(gs_plan* p, const double* h, double sealevel, double ofill, d
     p->pdir_bound = 0;
     // GS_TUNE_FLAT_BFS > 0 asks for the search over all depressions in tiles
     const bool all_at_once = p->bfs_window > 0;
-    if (all_at_once) GS_TRY(flat_compact(p, pit_ids));
-    // pit cells, compacted in id order for the flat pass and the per-pit reductions
-    GS_CUDA(cudaMemsetAsync(p->seg_count, 0, sizeof(int) * (np1 + 1), p->stream));
-    launch(p, k_pit_flag, G, B, n, (const int*)pit_ids, (const int*)p->spill_flag, p->pflag, p->seg_count, p->pdir);
-    GS_LAUNCH();
-    GS_TRY(exclusive_scan(p, p->pflag, p->pscan, n));
-    launch(p, k_pit_compact, G, B, n, (const int*)pit_ids, (const int*)p->pscan, p->seg_keys, p->seg_vals);
-    GS_LAUNCH();
-    int last[5] = {0, 0, 0, 0, 0};
+    int last[2] = {0, 0};
     if (all_at_once) {
+        GS_TRY(flat_compact(p, pit_ids));
         GS_CUDA(cudaMemcpyAsync(&last[0], p->scanbuf + n - 1, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
         GS_CUDA(cudaMemcpyAsync(&last[1], p->flagbuf + n - 1, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+        GS_CUDA(cudaStreamSynchronize(p->stream));
     }
-    GS_CUDA(cudaMemcpyAsync(&last[3], p->pscan + n - 1, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
-    GS_CUDA(cudaMemcpyAsync(&last[4], p->pflag + n - 1, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
-    GS_CUDA(cudaStreamSynchronize(p->stream));
-    const int ncell = last[3] + last[4];
     // pit cells sorted by (pit, id): segments for the flat pass and the per-pit
     // reductions.  The ordered compaction keeps id order; the stable radix sort
     // by pit then lists every pit's cells in increasing id.

@@ -79,3 +79,27 @@ def test_basin_levels_equal_the_priority_flood(kind, n, jitter, bc):
         assert np.array_equal(gm.lFill.cpu().numpy(), expect)
         assert pits is None or np.array_equal(gm.pitIDs.cpu().numpy(), pits)
     gm.destroy()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+def test_an_input_that_is_not_finite_leaves_the_fill_as_it_was(bad):
+    """The check is read with the fill's sizes, after its kernels have run."""
+    import torch
+    from gospl_b200 import synthetic as S
+    from gospl_b200.mesh import FVMesh
+    from gospl_b200.model import Model
+
+    coords, cells, z, rain, up, p = S.planar_config(n=3000, side=30.0e3, seed=3)
+    m = Model(coords=coords, cells=cells, elev=z, params=dict(p, rain=rain, upsub=up), mesh=FVMesh(coords, cells, p["bc"]),
+              device="cuda:0")
+    m.flowAccumulation()
+    keep = [x.clone() for x in (m.lFill, m.pitIDs, m.seaID, m.FAL)]
+    h0 = m.hGlobal.clone()
+    m.hGlobal[1234] = bad
+    with pytest.raises(Exception, match="non-finite"):
+        m.flowAccumulation()
+    assert torch.equal(m.lFill, keep[0]) and torch.equal(m.pitIDs, keep[1]) and torch.equal(m.seaID, keep[2])
+    m.hGlobal.copy_(h0)
+    m.flowAccumulation()
+    assert all(torch.equal(a, b) for a, b in zip((m.lFill, m.pitIDs, m.seaID, m.FAL), keep))
+    m.destroy()
