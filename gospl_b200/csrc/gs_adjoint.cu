@@ -209,7 +209,7 @@ int rec_pass_solve(gs_plan* p, int t, const int* order, int order_ok, const doub
     GS_TRY(rcopy(p, &q->rcv, (const int*)p->rcv, Rn));
     GS_TRY(rcopy(p, &q->wgt, (const double*)p->wgt, Rn));
     GS_TRY(rcopy(p, &q->rslot, (const int8_t*)p->rslot, Rn));
-    if (flow_needs_order(p)) GS_TRY(rcopy(p, &q->order, order, n));
+    if (flow_needs_order(p, TG_CASCADE)) GS_TRY(rcopy(p, &q->order, order, n));
     GS_TRY(rcopy(p, &q->x, x, n));
     return GS_OK;
 }

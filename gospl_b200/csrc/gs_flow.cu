@@ -275,8 +275,8 @@ static int read_flag(gs_plan* p, int* out) {
 }
 
 // outcome of a flow sweep whose status came back with a synchronisation
-static int flow_status(gs_plan* p, int st) {
-    if (!flow_needs_order(p)) return tile_status_check(p, st, "flow sweep did not complete");
+static int flow_status(gs_plan* p, int graph, int st) {
+    if (!flow_needs_order(p, graph)) return tile_status_check(p, st, "flow sweep did not complete");
     if (st != 0) set_error(st, "ordered flow sweep did not complete");
     return st;
 }
@@ -333,7 +333,7 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
     std::vector<uint8_t> lakes(nm, 0);
     GS_CUDA(cudaMemcpyAsync(lakes.data(), p->mlakes, nm, cudaMemcpyDeviceToHost, p->stream));
     GS_CUDA(cudaStreamSynchronize(p->stream));
-    GS_TRY(flow_status(p, *sweep_st));
+    GS_TRY(flow_status(p, TG_SNAP, *sweep_st));
     bool anyvol = false;
     for (int m = 0; m < nm; m++) anyvol = anyvol || lakes[m];
     int passes = 0, solves = 0;
@@ -369,7 +369,7 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
             GS_CUDA(cudaMemcpyAsync(p->h_mflags, p->mflags, sizeof(int) * nm, cudaMemcpyDeviceToHost, p->stream));
             GS_TRY(rec_pass_pits(p, step, lsink, np1));
             GS_CUDA(cudaStreamSynchronize(p->stream));
-            if (solving) GS_TRY(flow_status(p, *sweep_st));
+            if (solving) GS_TRY(flow_status(p, TG_CASCADE, *sweep_st));
             solving = false;
             int flags = 0;
             bool anybig = false, allbig = true;
@@ -402,7 +402,7 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
                 // receivers and the surface order do not need the flat BFS;
                 // the flat routing and the order's ties do: join it between
                 GS_TRY(receivers(p, p->R, 1.1, surf, sealevel, p->gid, p->rcv, p->dist, p->wgt, p->rslot));
-                if (flow_needs_order(p)) {
+                if (flow_needs_order(p, TG_CASCADE)) {
                     // the water surface differs from h only on lakes: reuse h's order
                     GS_TRY(flow_order_from(p, surf, h, p->order_i, p->order));
                     GS_TRY(flow_order_ties_prepare(p));
@@ -422,7 +422,7 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
                     launch(p, k_lsink_keep, G, B, n, (const int*)p->vmember, (const uint8_t*)p->mbig,
                            (const uint8_t*)p->lsink_prev, lsink);
                 GS_TRY(rec_pass_rebuild(p, step, surf));
-                if (flow_needs_order(p)) GS_TRY(flow_order_ties(p, p->pdir, p->order));
+                if (flow_needs_order(p, TG_CASCADE)) GS_TRY(flow_order_ties(p, p->pdir, p->order));
                 // the graph is prepared before the residual is read: one
                 // synchronisation gives the residual and the check
                 GS_TRY(flow_prepare(p, TG_CASCADE, p->rcv, p->wgt, p->rslot, p->q, surf, p->pdir, p->order,
@@ -474,7 +474,7 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
         }
         if (solving) {   // the loop ended right after a solve (pass limit, stagnation)
             GS_CUDA(cudaStreamSynchronize(p->stream));
-            GS_TRY(flow_status(p, *sweep_st));
+            GS_TRY(flow_status(p, TG_CASCADE, *sweep_st));
         }
         launch(p, k_lake_zero, G, B, n, h, (const double*)p->wf, (const int*)pit_ids, (const int*)p->vmember,
                (const uint8_t*)p->mlakes, fal);

@@ -126,6 +126,7 @@ struct gs_plan {
     // mesh tiles of the dataflow sweeps (gs_tiles.cu); tl_nt = 0: ordered sweeps
     bool mutual = true;                  // every edge is listed by both of its ends
     int tl_nt = 0;                       // tiles, one resident block each
+    int tl_cas = 0;                      // tiles that only TG_CASCADE is solved on (tl_nt = 0)
     int tl_T = 0;                        // vertices per tile
     int tl_np = 0;                       // predecessor slots of a record (6, 8 or 12)
     int tl_cap = 0;                      // most cut edges of a tile
@@ -139,7 +140,7 @@ struct gs_plan {
     unsigned* tl_cut_q = nullptr;        // position across each cut edge
     unsigned* tl_cut_l = nullptr;        // local vertex | slot << 16 of each cut edge
     uint16_t* tl_cut_idx = nullptr;      // [W][n] by position: cut edge of each slot within its tile
-    int tl_full = 0;                     // the whole records of a tile fit its block's shared memory
+    int tl_keep = 0;                     // records in shared memory: 2 whole, 1 their hot part, 0 none
     double* tl_xb = nullptr;             // [2][n] values published between tiles, two solves in turn
     unsigned* tl_status = nullptr;
     gs::TileGraph tl_graph[gs::TG_N];
@@ -333,7 +334,7 @@ int flow_order_from(gs_plan* p, const double* surface, const double* base_surfac
                     int* order);
 int flow_order_ties_prepare(gs_plan* p);   // after flow_order: tie groups of the surface
 int flow_order_ties(gs_plan* p, const int* pdir, int* order);   // after prepare: ties by pdir
-bool flow_needs_order(const gs_plan* p);   // the flow sweeps run in a vertex order (else on tiles)
+bool flow_needs_order(const gs_plan* p, int graph = TG_SNAP);   // its sweeps run in a vertex order (else on tiles)
 int flow_prepare(gs_plan* p, int graph, const int* rcv, const double* wgt, const int8_t* rslot, double* x,
                  const double* z, const int* pdir, const int* order, int* bad_host);
 // status_host (pinned): when given, the ordered sweep's status is copied

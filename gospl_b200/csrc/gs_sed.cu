@@ -671,15 +671,15 @@ int sed_change(gs_plan* p, double* h, double* cum_ed, const double* eb, const do
     int cyc = 0, total_cycles = 0;
     launch(p, k_sed_rhs, G, B, n, eb, (const double*)p->larea, p->q2);
     GS_LAUNCH();
-    GS_TRY(flow_prepare(p, TG_CASCADE, rcv_i, wgt_i, p->rslot_i, vsed, nullptr, nullptr, p->order_i,
+    GS_TRY(flow_prepare(p, TG_FLUX, rcv_i, wgt_i, p->rslot_i, vsed, nullptr, nullptr, p->order_i,
                         p->h_pinned + 3));
     int ok_i = p->order_i_valid;
-    if (!flow_needs_order(p)) {
+    if (!flow_needs_order(p, TG_FLUX)) {
         // (tiles: edges outside the checked snapshot graph take the counter-based sweep)
         GS_CUDA(cudaStreamSynchronize(p->stream));
         ok_i = ok_i && !p->h_pinned[3];
     }
-    GS_TRY(flow_run(p, TG_CASCADE, rcv_i, wgt_i, p->rslot_i, p->q2, vsed, &cyc, p->order_i, ok_i, nullptr));
+    GS_TRY(flow_run(p, TG_FLUX, rcv_i, wgt_i, p->rslot_i, p->q2, vsed, &cyc, p->order_i, ok_i, nullptr));
     total_cycles += cyc;
     // lsinki: sinks of the snapshot graph (flowplex.py:785-791)
     GS_TRY(sink_mask(p, wgt_i, sea, lsink));
@@ -760,7 +760,7 @@ int sed_change(gs_plan* p, double* h, double* cum_ed, const double* eb, const do
                 const double* surf = (step == 100) ? lfill : sfill;
                 rebuilt = true;
                 GS_TRY(receivers(p, p->R, 1.1, surf, sealevel, p->gid, p->rcv, p->dist, p->wgt, p->rslot));
-                if (flow_needs_order(p)) {
+                if (flow_needs_order(p, TG_CASCADE)) {
                     GS_TRY(flow_order_from(p, surf, hl, p->order_i, p->order));
                     GS_TRY(flow_order_ties_prepare(p));
                 }
@@ -772,7 +772,7 @@ int sed_change(gs_plan* p, double* h, double* cum_ed, const double* eb, const do
                            (const uint8_t*)p->lsink_prev, lsink);
                 // the tile graph is built with the rebuild (and kept over the
                 // passes that do not rebuild); its check comes back with the excess
-                if (flow_needs_order(p)) GS_TRY(flow_order_ties(p, p->pdir, p->order));
+                if (flow_needs_order(p, TG_CASCADE)) GS_TRY(flow_order_ties(p, p->pdir, p->order));
                 else
                     GS_TRY(flow_prepare(p, TG_CASCADE, p->rcv, p->wgt, p->rslot, routed, surf, p->pdir, p->order,
                                         p->h_pinned));
@@ -790,7 +790,7 @@ int sed_change(gs_plan* p, double* h, double* cum_ed, const double* eb, const do
                 GS_CUDA(cudaMemcpyAsync(p->msolve, solve.data(), nm, cudaMemcpyHostToDevice, p->stream));
                 if (!all(solve))
                     launch(p, k_rhs_members, G, B, n, (const int*)p->vmember, (const uint8_t*)p->msolve, nv);
-                if (flow_needs_order(p)) {
+                if (flow_needs_order(p, TG_CASCADE)) {
                     GS_TRY(flow_prepare(p, TG_CASCADE, p->rcv, p->wgt, p->rslot, routed, nullptr, nullptr, p->order,
                                         p->h_pinned));
                     GS_CUDA(cudaStreamSynchronize(p->stream));

@@ -28,6 +28,7 @@
 // edge against (surface, flat distance, id), a total order.  Every wait is
 // bounded by the plan's sweep budget (GS_ETIMEOUT).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -143,15 +144,21 @@ constexpr int HOT = 48;
 __host__ __device__ inline size_t tile_values(int T, int cut_cap) {
     return (((size_t)T + cut_cap) * 8 + 15) / 16 * 16;
 }
+// words of the counts: one each, or one for four vertices when no record is kept
+__host__ __device__ inline int tile_count_words(int T, bool bytes) {
+    return bytes ? (T + 7) / 8 * 2 : (T + 1) / 2 * 2;
+}
 __host__ __device__ inline size_t tile_smem(int T, int cut_cap, int rec_bytes) {
     const size_t t2 = (size_t)(T + 1) / 2 * 2;
-    return tile_values(T, cut_cap) + (size_t)T * rec_bytes + t2 * 4 + 128 + t2 * 2 + (size_t)cut_cap * 2;
+    return tile_values(T, cut_cap) + (size_t)T * rec_bytes + (size_t)tile_count_words(T, rec_bytes == 0) * 4 + 128 +
+           t2 * 2 + (size_t)cut_cap * 2;
 }
 
-// FULL: the tile's whole records are copied to shared memory first, else only
+// KEEP 2: the tile's whole records are copied to shared memory first; 1: only
 // their first HOT bytes and the divisors, and a vertex with more than four
-// predecessors or three successors reads the rest from L2.
-template <int NP, bool DIV, bool FULL>
+// predecessors or three successors reads the rest from L2; 0: none, every record
+// is read from L2 and a count takes a byte.
+template <int NP, bool DIV, int KEEP>
 __global__ void __launch_bounds__(TS_THREADS, 1) k_tile_sweep(SweepArgs a) {
     extern __shared__ double sm_tile[];
     __shared__ unsigned s_head, s_tail, s_ncut;
@@ -160,12 +167,14 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_tile_sweep(SweepArgs a) {
     const int T = a.T, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = TS_THREADS / 32, NWORK = NW - POLL_WARPS;   // warps that start with work
     const unsigned full = 0xffffffffu;
-    constexpr int RB = FULL ? R::BYTES : HOT;
+    constexpr bool FULL = KEEP == 2, HOTS = KEEP == 1;
+    constexpr int RB = FULL ? R::BYTES : HOTS ? HOT : 0;
     double* sx = sm_tile;
     char* srec = (char*)sm_tile + tile_values(T, a.cut_cap);
-    double* sdiv = (double*)(srec + (size_t)T * RB);   // without FULL
-    unsigned* cntw = (unsigned*)(sdiv + (FULL ? 0 : T));   // unsolved predecessors of l
-    unsigned* spare = cntw + (T + 1) / 2 * 2;
+    double* sdiv = (double*)(srec + (size_t)T * RB);   // with the hot parts
+    unsigned* cntw = (unsigned*)(sdiv + (HOTS ? T : 0));   // unsolved predecessors of l
+    const int nw = tile_count_words(T, KEEP == 0);
+    unsigned* spare = cntw + nw;
     unsigned short* queue = (unsigned short*)(spare + 32);
     unsigned short* act_cut = queue + (T + 1) / 2 * 2;
     volatile unsigned short* vq = queue;
@@ -195,18 +204,20 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_tile_sweep(SweepArgs a) {
         const unsigned f = a.pm[p];
         const unsigned nd = __popc(f & PM_PRED);
         sx[l] = a.b[a.perm ? a.perm[p] : p];
-        cntw[l] = nd;
+        if (KEEP == 0) ((uint8_t*)cntw)[l] = (uint8_t)nd;
+        else cntw[l] = nd;
         queue[l] = Q_EMPTY;
         if (DIV || nd || (f & (PM_IN | PM_OUT))) {
             work++;
-            if (!FULL && DIV) sdiv[l] = __ldg((const double*)(grec + (size_t)l * R::BYTES + R::OFF_DIV));
+            if (HOTS && DIV) sdiv[l] = __ldg((const double*)(grec + (size_t)l * R::BYTES + R::OFF_DIV));
         }
     }
     for (int e = tid; e < nc; e += TS_THREADS) sx[T + e] = __longlong_as_double((long long)XSENT);
-    for (int q = tid; q < m * (RB / 16); q += TS_THREADS) {
-        const int l = FULL ? 0 : q / (RB / 16), o = FULL ? q : q - l * (RB / 16);
-        ((uint4*)srec)[q] = __ldg((const uint4*)(grec + (size_t)l * R::BYTES) + o);
-    }
+    if constexpr (KEEP != 0)
+        for (int q = tid; q < m * (RB / 16); q += TS_THREADS) {
+            const int l = FULL ? 0 : q / (RB / 16), o = FULL ? q : q - l * (RB / 16);
+            ((uint4*)srec)[q] = __ldg((const uint4*)(grec + (size_t)l * R::BYTES) + o);
+        }
     if (tid < 32) spare[tid] = 0x40000000u;
     work = __reduce_add_sync(full, work);
     if (lane == 0 && work) atomicAdd(&s_left, work);
@@ -224,9 +235,13 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_tile_sweep(SweepArgs a) {
 
     // one predecessor of l solved: its count before
     const unsigned cnt_a = sm_addr(cntw), x_a = sm_addr(sx), rec_a = sm_addr(srec), div_a = sm_addr(sdiv);
-    auto arrive = [&](unsigned l) -> unsigned { return atoms_add(cnt_a + 4u * l, ~0u); };
+    auto arrive = [&](unsigned l) -> unsigned {
+        if (KEEP != 0) return atoms_add(cnt_a + 4u * l, ~0u);
+        const unsigned sh = 8u * (l & 3u);   // a count never goes below zero: no borrow
+        return (atoms_add(cnt_a + (l & ~3u), 0u - (1u << sh)) >> sh) & 0xffu;
+    };
     // absent successors count down a word of their lane that nothing reads
-    const unsigned none = (unsigned)((T + 1) / 2 * 2 + lane);
+    const unsigned none = (unsigned)(nw + lane) * (KEEP == 0 ? 4u : 1u);
     auto push = [&](unsigned l) {
         const unsigned pos = atomicAdd(&s_tail, 1u);   // a vertex is pushed at most once: pos < T
         vq[pos] = (unsigned short)l;
@@ -353,8 +368,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_tile_sweep(SweepArgs a) {
             const unsigned l = (unsigned)cur;
             const unsigned rs = rec_a + l * RB;
             const char* rg = grec + (size_t)l * R::BYTES;
-            const uint4 hd = lds_u128(rs);
-            const double2 w01 = lds_2f64(rs + R::OFF_W), w23 = lds_2f64(rs + R::OFF_W + 16);
+            const uint4 hd = KEEP != 0 ? lds_u128(rs) : __ldg((const uint4*)rg);
+            const double2 w01 = KEEP != 0 ? lds_2f64(rs + R::OFF_W) : __ldg((const double2*)(rg + R::OFF_W)),
+                          w23 = KEEP != 0 ? lds_2f64(rs + R::OFF_W + 16) : __ldg((const double2*)(rg + R::OFF_W + 16));
             const double dv = !DIV ? 1.0 : FULL ? lds_f64(rs + R::OFF_DIV) : lds_f64(div_a + 8u * l);
             const unsigned info = hd.y >> 16;
             const int nd = (int)(info & RI_ND), ns = (int)((info >> RI_NS_SHIFT) & 0xfu);
@@ -701,9 +717,10 @@ int by_width(const gs_plan* p, F f) {
 }
 
 template <int NP>
-const void* sweep_kernel(bool div, bool whole) {
-    if (whole) return div ? (const void*)k_tile_sweep<NP, true, true> : (const void*)k_tile_sweep<NP, false, true>;
-    return div ? (const void*)k_tile_sweep<NP, true, false> : (const void*)k_tile_sweep<NP, false, false>;
+const void* sweep_kernel(bool div, int keep) {
+    if (keep == 2) return div ? (const void*)k_tile_sweep<NP, true, 2> : (const void*)k_tile_sweep<NP, false, 2>;
+    if (keep == 1) return div ? (const void*)k_tile_sweep<NP, true, 1> : (const void*)k_tile_sweep<NP, false, 1>;
+    return div ? nullptr : (const void*)k_tile_sweep<NP, false, 0>;
 }
 
 }  // namespace
@@ -773,10 +790,13 @@ static void grow_tiles(int n, const int32_t* nnb, const int32_t* ngb, int T, std
 // (rows of a lattice, mesh generators) get grown tiles.
 // A tile must fit its block's shared memory with the hot part of its records
 // (about 3,200 vertices a tile, 460,000 in all).  Larger meshes keep the
-// ordered sweeps (tl_nt = 0): with records left in L2 a tile solves about 100
+// ordered sweeps (tl_nt = 0) but for the cascade's flow (tl_cas), which would
+// have to merge an order first: with records left in L2 a tile solves about 100
 // vertices/us and a hop takes 0.65 us, and the two flow sweeps of a step took
-// 260 + 350 us at 655,362 vertices and 740 + 780 us at 2,621,442, against 380 +
-// 820 us in the ordered form there.
+// 260 + 350 us at 655,362 vertices and 740 + 1,060 us at 2,621,442, against 380 +
+// 820 us in the ordered form there (flow_needs_order).  Loading the first
+// successor's record ahead made it 10 % slower: the fences wait for it.  Values, a byte of count
+// and a queue slot per vertex fit for 2.7 million vertices.
 // Not called for a mesh with an edge that only one of its ends lists (a vertex
 // of more than twelve neighbours, of which the reference keeps the first
 // twelve): solved vertices are announced through the neighbour lists.
@@ -791,12 +811,21 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
     const int blocks = std::max(p->sm_count - SM_SPARE, 1);
     const int64_t per = ((int64_t)n + blocks - 1) / blocks;
     const int64_t T64 = std::max<int64_t>(TILE_MIN, (per + 31) / 32 * 32);
-    if (T64 > TILE_MAX || tile_smem((int)T64, 0, HOT + 8) > room) return GS_OK;
+    if (T64 > TILE_MAX || tile_smem((int)T64, 0, 0) > room) return GS_OK;
     const int T = (int)T64;
+    const bool cas = tile_smem(T, 0, HOT + 8) > room;   // the cascade's flow alone
     const int nt = (n + T - 1) / T;
     std::vector<int> perm, loc, cuts, gcuts;
     count_cuts(n, nnb, ngb, T, nt, nullptr, cuts);
-    if (nt > 1) {
+    if (cas) {
+        // consecutive ids as they are, or not at all: growing tiles of so many
+        // vertices costs the host more than many steps save.  A compact patch cuts
+        // about 8 sqrt(T) edges, one along a space-filling curve up to twice that,
+        // the strips of a lattice's rows some 60 sqrt(T).
+        int64_t total = 0;
+        for (int c : cuts) total += c;
+        if ((double)total > 24.0 * sqrt((double)T) * nt) return GS_OK;
+    } else if (nt > 1) {
         grow_tiles(n, nnb, ngb, T, perm);
         // by id within a tile: neighbours in memory stay together
         for (int t = 0; t < nt; t++)
@@ -840,11 +869,11 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
     int ok = 1;
     by_width(p, [&](auto w) -> int {
         constexpr int NP = decltype(w)::value;
-        p->tl_full = tile_smem(T, cap, Rec<NP>::BYTES) <= room;
-        p->tl_smem = tile_smem(T, cap, p->tl_full ? Rec<NP>::BYTES : HOT + 8);
+        p->tl_keep = cas ? 0 : tile_smem(T, cap, Rec<NP>::BYTES) <= room ? 2 : 1;
+        p->tl_smem = tile_smem(T, cap, p->tl_keep == 2 ? Rec<NP>::BYTES : p->tl_keep == 1 ? HOT + 8 : 0);
         if (p->tl_smem > room) ok = 0;
-        for (int div = 0; div < 2 && ok; div++) {
-            const void* k = sweep_kernel<NP>(div != 0, p->tl_full != 0);
+        for (int div = 0; div < (cas ? 1 : 2) && ok; div++) {
+            const void* k = sweep_kernel<NP>(div != 0, p->tl_keep);
             int o = 0;
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->tl_smem) != cudaSuccess ||
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, TS_THREADS, p->tl_smem) != cudaSuccess || o < 1)
@@ -876,7 +905,7 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
                  o_pm = put(perm.data(), lp ? sizeof(int) * N : 0), o_lc = put(loc.data(), lp ? sizeof(int) * N : 0);
     const size_t o_xb = host.size(), o_g = o_xb + (2 * N * sizeof(double) + 31) / 32 * 32;
     const size_t g_bytes = rec_bytes + (N * sizeof(uint16_t) + 31) / 32 * 32;
-    cudaError_t e = cudaMalloc((void**)&p->tl_pool, o_g + TG_N * g_bytes);
+    cudaError_t e = cudaMalloc((void**)&p->tl_pool, o_g + (cas ? 1 : TG_N) * g_bytes);
     if (e != cudaSuccess) {
         p->tl_pool = nullptr;
         cudaGetLastError();
@@ -893,18 +922,20 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
     p->tl_loc = lp ? (int*)(p->tl_pool + o_lc) : nullptr;
     p->tl_xb = (double*)(p->tl_pool + o_xb);
     for (int g = 0; g < TG_N; g++) {
-        p->tl_graph[g].rec = p->tl_pool + o_g + g * g_bytes;
+        if (cas && g != TG_CASCADE) continue;
+        p->tl_graph[g].rec = p->tl_pool + o_g + (cas ? 0 : g) * g_bytes;
         p->tl_graph[g].pm = (uint16_t*)(p->tl_graph[g].rec + rec_bytes);
     }
     p->tl_dirty = 1;
-    p->tl_nt = nt;
+    p->tl_nt = cas ? 0 : nt;
+    p->tl_cas = cas ? nt : 0;
     return GS_OK;
 }
 
 void tiles_free(gs_plan* p) {
     if (p->tl_pool) cudaFree(p->tl_pool);
     p->tl_pool = nullptr;
-    p->tl_nt = 0;
+    p->tl_nt = p->tl_cas = 0;
 }
 
 static BuildArgs build_args(gs_plan* p, const TileGraph& g) {
@@ -990,13 +1021,13 @@ int tile_solve(gs_plan* p, int which, bool div, const double* b, double* x, cons
     p->tl_par = 1 - p->tl_par;
     return by_width(p, [&](auto w) -> int {
         constexpr int NP = decltype(w)::value;
-        const void* fn = sweep_kernel<NP>(div, p->tl_full != 0);
+        const void* fn = sweep_kernel<NP>(div, p->tl_keep);
         void* args[] = {(void*)&a};
         GS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->tl_smem));
         cudaEvent_t stop = nullptr;
         if (p->profiling) prof_begin(p, fn, &stop);
         // the blocks wait on one another: a cooperative launch keeps them all resident
-        GS_CUDA(cudaLaunchCooperativeKernel(fn, p->tl_nt, TS_THREADS, args, p->tl_smem, p->stream));
+        GS_CUDA(cudaLaunchCooperativeKernel(fn, std::max(p->tl_nt, p->tl_cas), TS_THREADS, args, p->tl_smem, p->stream));
         if (stop) cudaEventRecord(stop, p->stream);
         p->launches++;
         return GS_OK;

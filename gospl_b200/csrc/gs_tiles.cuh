@@ -17,8 +17,11 @@ struct TileGraph {
 // edges passed the acyclicity check; TG_CASCADE: any other donors-first graph;
 // TG_UP: receivers-first graphs
 enum { TG_SNAP = 0, TG_CASCADE = 1, TG_UP = 2, TG_N = 3 };
+// the snapshot graph's edges with other weights, in TG_CASCADE's records
+enum { TG_FLUX = TG_N };
 
-// the plan's tiles (tl_nt = 0 when the mesh keeps the ordered sweeps)
+// the plan's tiles (tl_nt = 0 when the mesh keeps the ordered sweeps; tl_cas > 0:
+// but for the cascade's flow)
 int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb);
 void tiles_free(gs_plan* p);
 // Records of graph `which` from the receiver edges rcv/rslot with a non-zero

@@ -81,3 +81,34 @@ def test_flow_and_spl_sweeps_equal_the_sequential_solves(kind, n, R):
     E[m.lsink.cpu().numpy()] = 0.0
     assert np.array_equal(m.hGlobal.cpu().numpy(), h0 + E * 1000.0)
     m.destroy()
+
+
+@pytest.mark.parametrize("level,R,sed", [(7, 3, True), (8, 3, True), (8, 1, False), (8, 6, False)])
+def test_cascade_on_tiles_equals_the_ordered_sweeps(level, R, sed):
+    """Above the size whose records fit shared memory the cascade's flow alone is
+    solved on tiles; a model that records for the adjoint takes the ordered
+    sweeps there.  Donors are added in ascending id on both: equal bit for bit
+    (below that size both models run the same tiles)."""
+    import torch
+    from gospl_b200 import _lib
+    from gospl_b200 import synthetic as S
+    from gospl_b200.mesh import FVMesh
+    from gospl_b200.model import Model
+    coords, cells, z, rain, up, p = S.sphere_config(level=level, lmax=128)
+    p = dict(p, rain=rain, upsub=up, flowDir=R, nodep=not sed, nlPitVolume=float("inf"))
+    fv = FVMesh(coords, cells, p["bc"], device="cuda:0")
+    out = []
+    for recorded in (False, True):
+        m = Model(coords=coords, cells=cells, elev=z, params=p, mesh=fv, device="cuda:0")
+        if recorded:
+            _lib.check(_lib.load().gs_plan_record(m._plan, 1))
+        m.flowAccumulation()
+        assert m.stats["flow"]["cascade_solves"] > 0
+        if sed:
+            m.erodepSPL()
+            m.flowAccumulation()
+            m.sedChange()
+            assert m.stats["sed"]["cascade_solves"] > 0
+        out.append([x.clone() for x in (m.FAL, m.fillFAL, m.waterFilled, m.hGlobal)])
+        m.destroy()
+    assert all(torch.equal(a, b) for a, b in zip(*out))
