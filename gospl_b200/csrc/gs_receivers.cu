@@ -12,6 +12,8 @@
 //
 // k_flow_direction_post restates flowplex.py:480-540: flat routing on filled
 // pits when down=True, self-sink outlets on flat models, the lsink mask.
+#include <type_traits>
+
 #include "gs_plan.cuh"
 
 namespace gs {
@@ -177,29 +179,133 @@ __global__ void k_mfd_receivers(int n, int W, int R, double expo, const double* 
     if (k < n) mfd_vertex_general(k, n, R, expo, elev, sl, gid, nbr, elen, nnb, rcv, dist, wgt, rslot);
 }
 
-// Register form for R = RM <= 4 (the configurations' flowDir is 3), in two
-// passes over the neighbour slots so that no per-slot array is held: the
-// first finds the steepest gradient (the exponent), the second forms every
-// candidate slope, sums them in slot order and keeps the RM + 1 steepest by
-// insertion.  The second pass re-reads the slot's id, edge length and the
-// neighbour's elevation (L1/L2 hits) instead of keeping 12 of each in
-// registers, which keeps the kernel near 64 registers and the SMs full of
-// warps for the gathers.  Without exact ties among the kept candidates the
-// descending order is the one the reference quicksort leaves, so the result
-// is bit-identical to the general form; a vertex whose new candidate equals a
-// kept one goes to mfd_vertex_general (literal replay).  gid == nullptr means
-// the identity numbering (one partition).
-template <int RM>
-__global__ void __launch_bounds__(128) k_mfd_receivers_r(int n, double expo, const double* __restrict__ elev,
+// What k_flow_direction_post does to the receivers of the unfilled surface, in
+// the kernel that finds them: outlets of flat models drain to themselves (flat),
+// and the masks when they are asked for (lsink).
+struct DirPost {
+    const uint8_t* flat = nullptr;      // outlet flags, null: none drain to themselves
+    const uint8_t* outlet = nullptr;
+    const double* lfill = nullptr;
+    uint8_t* lsink = nullptr;
+    uint8_t* sea = nullptr;
+};
+__device__ __forceinline__ void dir_masks(const DirPost& post, int k, double sl, bool none) {
+    if (!post.lsink) return;
+    const bool is_sea = post.lfill[k] <= sl;
+    post.lsink[k] = (none && !post.outlet[k] && !is_sea) ? 1 : 0;
+    post.sea[k] = is_sea ? 1 : 0;
+}
+
+// neighbours c (-1: none), edge lengths l and drops d of a vertex, all gathers
+// in flight together, and the exponent from its steepest gradient
+template <int NP>
+__device__ __forceinline__ void mfd_gather(int k, int n, double hk, const double* __restrict__ elev,
+                                           const int* __restrict__ nbr, const double* __restrict__ elen,
+                                           const int8_t* __restrict__ nnb, double expo, int (&c)[NP], double (&l)[NP],
+                                           double (&d)[NP], double& fexp) {
+    const int deg = nnb[k];
+#pragma unroll
+    for (int s = 0; s < NP; s++) {
+        c[s] = s < deg ? nbr[(size_t)s * n + k] : -1;
+        l[s] = s < deg ? elen[(size_t)s * n + k] : 0.0;
+    }
+#pragma unroll
+    for (int s = 0; s < NP; s++) d[s] = c[s] >= 0 ? hk - elev[c[s]] : 0.0;
+    double e = 0.0;
+#pragma unroll
+    for (int s = 0; s < NP; s++) {
+        if (!(l[s] > 0.0)) c[s] = -1;
+        if (c[s] < 0) continue;
+        const double g = d[s] / l[s];
+        e = (g > e) ? g : e;
+    }
+    fexp = e > 0 ? 5.0 * ((e < 1.0) ? e : 1.0) + expo : 1.0;
+}
+
+__device__ __forceinline__ double mfd_slope(double d, double l, double fexp, bool fexp_int) {
+    if (d > 0.0) return pow(d, fexp) / l;
+    if (d == 0.0) return 0.0;
+    return fexp_int ? pow(d, fexp) / l : -1.0;   // non-integer power of a negative base is NaN
+}
+
+// R >= the mesh's neighbour slots: every candidate is a receiver, in slot order,
+// and nothing has to be ranked.  The powers of the land vertices bound it, then
+// the stores: eight directions of 655,362 vertices and their masks take 56 us,
+// where the general form (arrays in local memory) and a pass for the masks took
+// 73.  Six slots: 64 registers for eight blocks an SM, 4 % faster than 78.
+template <int NP>
+__global__ void __launch_bounds__(128, NP == 6 ? 8 : 1) k_mfd_all(int n, int R, double expo, const double* __restrict__ elev,
+                                                  double sl, const int* __restrict__ gid, const int* __restrict__ nbr,
+                                                  const double* __restrict__ elen, const int8_t* __restrict__ nnb,
+                                                  int* __restrict__ rcv, double* __restrict__ dist,
+                                                  double* __restrict__ wgt, int8_t* __restrict__ rslot,
+                                                  const DirPost post) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const double hk = elev[k];
+    int c[NP], kk = 0;
+    double l[NP], x[NP], tot = 0.0;
+    unsigned mask = 0u;
+    if (!(hk <= sl) && !(post.flat && post.flat[k])) {
+        double d[NP], fexp;
+        mfd_gather<NP>(k, n, hk, elev, nbr, elen, nnb, expo, c, l, d, fexp);
+        const bool fexp_int = (fexp == floor(fexp));
+#pragma unroll
+        for (int s = 0; s < NP; s++) {
+            x[s] = 0.0;
+            if (c[s] < 0) continue;
+            const double val = mfd_slope(d[s], l[s], fexp, fexp_int);
+            if (!(val > 0.0)) continue;
+            x[s] = val * (1.0 - 1.0e-15 * (double)(gid ? gid[c[s]] : c[s]));
+            tot = tot + x[s];
+            mask |= 1u << s;
+            kk++;
+        }
+    }
+    double sw = 0.0;
+    for (int o = 0; o < R; o++) {
+        int r = k, slot = -1;
+        double dd = 0.0, w = 0.0;
+        if (o < kk) {
+            slot = __ffs(mask) - 1;
+            mask &= mask - 1u;
+#pragma unroll
+            for (int s = 0; s < NP; s++)
+                if (s == slot) {
+                    r = c[s];
+                    dd = l[s];
+                    w = x[s] / tot;
+                }
+        }
+        rcv[(size_t)o * n + k] = r;
+        dist[(size_t)o * n + k] = dd;
+        wgt[(size_t)o * n + k] = w;
+        sw = sw + w;
+        if (rslot) rslot[(size_t)o * n + k] = (int8_t)slot;
+    }
+    dir_masks(post, k, sl, sw == 0.0);
+}
+
+// Register form for R = RM < the neighbour slots NP: every candidate slope is
+// formed and summed in slot order, and the RM + 1 steepest are kept by
+// insertion.  Without exact ties among the kept candidates the descending order
+// is the one the reference quicksort leaves, so the result is bit-identical to
+// the general form; a vertex whose new candidate equals a kept one goes to
+// mfd_vertex_general (literal replay).  gid == nullptr means the identity
+// numbering (one partition).  The gathers of a vertex are in flight together: in
+// a loop over its slots, and once more in the second pass over them, three
+// directions took 22 us on 20,000 vertices and 125 on 2.6 million, now 18 and 112.
+template <int RM, int NP>
+__global__ void __launch_bounds__(128, NP == 6 ? 8 : 1) k_mfd_receivers_r(int n, double expo, const double* __restrict__ elev,
                                                           double sl, const int* __restrict__ gid,
                                                           const int* __restrict__ nbr, const double* __restrict__ elen,
                                                           const int8_t* __restrict__ nnb, int* __restrict__ rcv,
                                                           double* __restrict__ dist, double* __restrict__ wgt,
-                                                          int8_t* __restrict__ rslot) {
+                                                          int8_t* __restrict__ rslot, const DirPost post) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const double hk = elev[k];
-    if (!(hk > sl)) {
+    if (!(hk > sl) || (post.flat && post.flat[k])) {
 #pragma unroll
         for (int o = 0; o < RM; o++) {
             rcv[(size_t)o * n + k] = k;
@@ -207,25 +313,12 @@ __global__ void __launch_bounds__(128) k_mfd_receivers_r(int n, double expo, con
             wgt[(size_t)o * n + k] = 0.0;
             if (rslot) rslot[(size_t)o * n + k] = -1;
         }
+        dir_masks(post, k, sl, true);
         return;
     }
-    const int deg = nnb[k];
-    double e = 0.0;
-    for (int s = 0; s < deg; s++) {
-        const int c = nbr[(size_t)s * n + k];
-        const double l = elen[(size_t)s * n + k];
-        if (c >= 0 && l > 0.0) {
-            const double g = (hk - elev[c]) / l;
-            e = (g > e) ? g : e;
-        }
-    }
-    double fexp;
-    if (e > 0) {
-        const double me = (e < 1.0) ? e : 1.0;
-        fexp = 5.0 * me + expo;
-    } else {
-        fexp = 1.0;
-    }
+    int c[NP];
+    double l[NP], d[NP], fexp;
+    mfd_gather<NP>(k, n, hk, elev, nbr, elen, nnb, expo, c, l, d, fexp);
     const bool fexp_int = (fexp == floor(fexp));
     // candidates: slope (scaled by the global-id tie-break), kept descending;
     // strict > keeps the earlier slot ahead of an equal value
@@ -241,21 +334,16 @@ __global__ void __launch_bounds__(128) k_mfd_receivers_r(int n, double expo, con
     int kk = 0;
     double tot_all = 0.0;
     bool tie = false;
-    for (int s = 0; s < deg; s++) {
-        const int c = nbr[(size_t)s * n + k];
-        const double l = elen[(size_t)s * n + k];
-        if (c < 0 || !(l > 0.0)) continue;
-        const double d = hk - elev[c];
-        double val;
-        if (d > 0.0) val = pow(d, fexp) / l;
-        else if (d == 0.0) val = 0.0;
-        else val = fexp_int ? pow(d, fexp) / l : -1.0;   // non-integer power of a negative base is NaN
+#pragma unroll
+    for (int s = 0; s < NP; s++) {
+        if (c[s] < 0) continue;
+        const double val = mfd_slope(d[s], l[s], fexp, fexp_int);
         if (!(val > 0.0)) continue;
-        double x = val * (1.0 - 1.0e-15 * (double)(gid ? gid[c] : c));
+        double x = val * (1.0 - 1.0e-15 * (double)(gid ? gid[c[s]] : c[s]));
         mask |= 1u << s;
         kk++;
         tot_all = tot_all + x;
-        int xs = s, xi = c;
+        int xs = s, xi = c[s];
 #pragma unroll
         for (int j = 0; j <= RM; j++) tie |= (x == tv[j]);
 #pragma unroll
@@ -272,6 +360,7 @@ __global__ void __launch_bounds__(128) k_mfd_receivers_r(int n, double expo, con
             }
         }
     }
+    double sw = 0.0;
     if (kk <= RM) {
         // every candidate is kept: receivers in slot order, weights over the
         // sum of all candidates taken in slot order
@@ -283,7 +372,9 @@ __global__ void __launch_bounds__(128) k_mfd_receivers_r(int n, double expo, con
                 for (int i = 0; i < RM; i++) o += (i < kk && ts[i] < ts[j]) ? 1 : 0;
                 rcv[(size_t)o * n + k] = tid[j];
                 dist[(size_t)o * n + k] = elen[(size_t)ts[j] * n + k];
-                wgt[(size_t)o * n + k] = tv[j] / tot_all;
+                const double w = tv[j] / tot_all;
+                sw = sw + w;
+                wgt[(size_t)o * n + k] = w;
                 if (rslot) rslot[(size_t)o * n + k] = (int8_t)ts[j];
             } else {
                 rcv[(size_t)j * n + k] = k;
@@ -292,10 +383,14 @@ __global__ void __launch_bounds__(128) k_mfd_receivers_r(int n, double expo, con
                 if (rslot) rslot[(size_t)j * n + k] = -1;
             }
         }
+        dir_masks(post, k, sl, sw == 0.0);
         return;
     }
     if (tie) {
         mfd_vertex_general(k, n, RM, expo, elev, sl, gid, nbr, elen, nnb, rcv, dist, wgt, rslot);
+        if (post.lsink)
+            for (int o = 0; o < RM; o++) sw = sw + wgt[(size_t)o * n + k];
+        dir_masks(post, k, sl, sw == 0.0);
         return;
     }
     // reference quirk: receiver o takes the edge length of candidate kk-1-o
@@ -311,9 +406,12 @@ __global__ void __launch_bounds__(128) k_mfd_receivers_r(int n, double expo, con
         m &= ~(1u << hs);
         rcv[(size_t)o * n + k] = tid[o];
         dist[(size_t)o * n + k] = elen[(size_t)hs * n + k];
-        wgt[(size_t)o * n + k] = tv[o] / tot;
+        const double w = tv[o] / tot;
+        sw = sw + w;
+        wgt[(size_t)o * n + k] = w;
         if (rslot) rslot[(size_t)o * n + k] = (int8_t)ts[o];
     }
+    dir_masks(post, k, sl, sw == 0.0);
 }
 
 __global__ void k_flow_direction_post(int n, int W, int R, int flat, const double* __restrict__ h,
@@ -387,32 +485,56 @@ int sink_mask(gs_plan* p, const double* wgt, const uint8_t* sea, uint8_t* lsink)
     return GS_OK;
 }
 
-int receivers(gs_plan* p, int nrcv, double exp, const double* elev, double sl, const int* gid,
-              int* rcv, double* dist, double* wgt, int8_t* rslot) {
+// `post` runs in the receivers' kernel where *fused comes back true
+static int receivers_post(gs_plan* p, int nrcv, double exp, const double* elev, double sl, const int* gid, int* rcv,
+                          double* dist, double* wgt, int8_t* rslot, const DirPost& post, bool* fused) {
     if (nrcv < 1 || nrcv > 12) {
         set_error(GS_EINVAL, "mfdreceivers: nrcv must be in 1..12");
         return GS_EINVAL;
     }
+    *fused = nrcv >= p->W || nrcv <= 4;
     if (p->n == 0) return GS_OK;
     const int* g = gid == p->gid ? nullptr : gid;   // the plan's own numbering is the identity
     const int G = grid_for(p->n, 128), n = (int)p->n;
-    switch (nrcv) {
-        case 1: launch(p, k_mfd_receivers_r<1>, G, 128, n, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt, rslot); break;
-        case 2: launch(p, k_mfd_receivers_r<2>, G, 128, n, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt, rslot); break;
-        case 3: launch(p, k_mfd_receivers_r<3>, G, 128, n, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt, rslot); break;
-        case 4: launch(p, k_mfd_receivers_r<4>, G, 128, n, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt, rslot); break;
-        default:
-            launch(p, k_mfd_receivers, G, 128, n, p->W, nrcv, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist,
-                   wgt, rslot);
-    }
+    // slots of the unrolled forms (6: spheres, 8: jittered lattices, 12)
+    auto width = [&](auto f) {
+        if (p->W <= 6) f(std::integral_constant<int, 6>{});
+        else if (p->W <= 8) f(std::integral_constant<int, 8>{});
+        else f(std::integral_constant<int, 12>{});
+    };
+    if (nrcv >= p->W)
+        width([&](auto w) {
+            launch(p, k_mfd_all<decltype(w)::value>, G, 128, n, nrcv, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv,
+                   dist, wgt, rslot, post);
+        });
+    else if (nrcv <= 4)
+        width([&](auto w) {
+            constexpr int NP = decltype(w)::value;
+            launch(p, nrcv == 1 ? k_mfd_receivers_r<1, NP> : nrcv == 2 ? k_mfd_receivers_r<2, NP>
+                      : nrcv == 3 ? k_mfd_receivers_r<3, NP> : k_mfd_receivers_r<4, NP>,
+                   G, 128, n, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt, rslot, post);
+        });
+    else
+        launch(p, k_mfd_receivers, G, 128, n, p->W, nrcv, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt,
+               rslot);
     GS_LAUNCH();
     return GS_OK;
+}
+
+int receivers(gs_plan* p, int nrcv, double exp, const double* elev, double sl, const int* gid,
+              int* rcv, double* dist, double* wgt, int8_t* rslot) {
+    bool fused;
+    return receivers_post(p, nrcv, exp, elev, sl, gid, rcv, dist, wgt, rslot, DirPost{}, &fused);
 }
 
 int flow_direction(gs_plan* p, const double* h, bool down, const double* lfill, const int* pit_ids,
                    const int* flat_dirs, double sealevel, int* rcv, double* dist, double* wgt,
                    int8_t* rslot, uint8_t* lsink, uint8_t* sea) {
-    GS_TRY(receivers(p, p->R, 1.1, h, sealevel, p->gid, rcv, dist, wgt, rslot));
+    DirPost post;
+    if (!down) post = DirPost{p->flat ? p->outlet : nullptr, p->outlet, lfill, lsink, sea};
+    bool fused = false;
+    GS_TRY(receivers_post(p, p->R, 1.1, h, sealevel, p->gid, rcv, dist, wgt, rslot, post, &fused));
+    if (fused && !down) return GS_OK;
     return flow_direction_post(p, h, down, lfill, pit_ids, flat_dirs, sealevel, rcv, dist, wgt, rslot, lsink, sea);
 }
 
