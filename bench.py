@@ -985,6 +985,8 @@ def _short(name):
         return "k_dataflow_flow" if "FlowOp" in s else ("k_dataflow_spl" if "SplOp" in s else "k_dataflow")
     if "k_mfd_receivers" in s:
         return "k_mfd_receivers"
+    if "k_tile_sweep" in s:
+        return "k_tile_sweep"
     for tok in s.replace("(", " ").replace("<", " ").split():
         if tok.startswith("_ZN2gs"):
             rest = tok[6:]
@@ -1029,6 +1031,10 @@ def algo_bytes_per_launch(kname, L):
     if kname == "k_ordered_spl":
         # order 4, rcv 4R, coefficient 8R, hOld 8, h write 8
         return n * (4 + 12 * R + 16)
+    if kname == "k_tile_sweep":
+        # predecessor slots 2, b 8, x write 8, record head 16; per link:
+        # weight 8, predecessor and successor ids 2 + 2
+        return n * (2 + 8 + 8 + 16) + E * (8 + 2 + 2)
     if kname in ("k_bfs_local", "k_bfs_tiles"):
         # packed rows of the pit cells (count + up to W local ids, padded to
         # a multiple of 4 ints) and one distance write per cell

@@ -10,8 +10,8 @@
 //   1. steepest non-ascending descent (lexicographic (z, id)) links every cell
 //      to a root: a seed or a local minimum (a basin);
 //   2. for each pair of adjacent basins the spill height is max(z_u, z_v);
-//   3. basin levels L(b) = minimax over basin-graph paths to a seed basin,
-//      relaxed with atomicMin until stable;
+//   3. basin levels L(b) = minimax over basin-graph paths to a seed basin, by
+//      contracting the graph along the components' lowest edges;
 //   4. fill = max(z, L(basin)).
 // Only comparisons are involved, so the result is bit-identical to the
 // reference's heap-ordered flood.  Seeds and exclusions follow edge_tile
@@ -22,8 +22,8 @@
 // Pit bookkeeping follows _pitInformation (pitfilling.py:704-847):
 // label_pits (equal-fill components holding a cell with no lower neighbour,
 // numbered by their smallest seed id) by union-find; pits_cons renumbering;
-// spill selection by smallest id; fill_dir / nghb_dir hop distances by
-// level-synchronous BFS; the (distance, id) flat receiver pick; pit volumes,
+// spill selection by smallest id; fill_dir / nghb_dir hop distances by a
+// search in each depression; the (distance, id) flat receiver pick; pit volumes,
 // depths and depth-volume curves (_getPitParams, getpitvol) by deterministic
 // segmented reductions over pit-sorted cells.
 #include <cub/cub.cuh>

@@ -6,6 +6,10 @@
 // Stream-power erosion (SPL.py:45-114, solved at SPL.py:297):
 //     h_i = (hOld_i + sum_k c_ik h_{rcv_ik}) / (1 + sum_k c_ik).
 //
+// Which form a call takes is said at flow_needs_order: mesh tiles (gs_tiles.cu),
+// the ordered sweep (k_ordered below), or the counter-based one described here
+// where an order or a tile graph fails its check.
+//
 // Both are solved exactly in one pass: each vertex carries a count of its
 // unresolved predecessors; vertices whose count reaches zero are appended to
 // a ready queue; a persistent grid pulls tickets from the queue, computes the

@@ -94,9 +94,9 @@ int gs_plan_set_stream(gs_plan* plan, void* cuda_stream);
 #define GS_TUNE_SWEEP_NAP 5       /* longest back-off between polls of the ordered sweeps, ns (0..1024, default 32) */
 #define GS_TUNE_SWEEP_BUDGET 6    /* wall-clock budget of one dependency sweep, us (1..6e7, default 4e6): a sweep
                                      still waiting on a predecessor after it stops with GS_ETIMEOUT */
-#define GS_TUNE_FLAT_BFS 7        /* flat-distance BFS: 0 one block with the visited set in shared memory
-                                     (default; tiles when the set does not fit), w in 1..4096 tiles in one
-                                     cooperative launch settling distance windows of w levels */
+#define GS_TUNE_FLAT_BFS 7        /* flat-distance search: 0 by depression (default), w in 1..4096 over all
+                                     depressions in tiles, one cooperative launch settling distance windows
+                                     of w levels */
 #define GS_TUNE_WARM_START 8      /* 1 (default): the hillslope CG starts from h plus the previous step's
                                      diffusion change and the bathymetry smoothing from the previous
                                      smoothing; 0: both start from their right-hand side, so that a step
