@@ -292,6 +292,11 @@ int flow_accumulation(gs_plan* p, const double* h, const double* bl, double seal
     // fill) and the topological order of their graph, on side_a while the
     // main stream fills depressions.
     int* bad_a = p->h_pinned + 1;
+    const int tiles = flow_needs_order(p) ? 0 : 1;
+    if (tiles != p->snap_tiles) {   // the other form's check says nothing about this one's
+        p->snap_tiles = tiles;
+        p->order_i_valid = 0;
+    }
     GS_CUDA(cudaEventRecord(p->ev_fork_a, p->stream));
     GS_CUDA(cudaStreamWaitEvent(p->side_a, p->ev_fork_a, 0));
     {

@@ -61,6 +61,11 @@ static void plan_free(gs_plan* p) {
     if (p->h_pinned) cudaFreeHost(p->h_pinned);
 }
 
+__global__ void k_identity(int n, int* a) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) a[i] = i;
+}
+
 int plan_create(int64_t nb, const int32_t* nnb, const int32_t* ngb, const double* elgt, const double* vdist,
                 const double* farea, const double* larea, const int32_t* outlet_ids, int64_t n_outlet,
                 const int32_t* open_ids, int64_t n_open, int flat, int flow_dir, gs_plan** out) {
@@ -205,6 +210,8 @@ int plan_create(int64_t nb, const int32_t* nnb, const int32_t* ngb, const double
         TRYP(dalloc(&p->q3, N));
         TRYP(dalloc(&p->order, N));
         TRYP(dalloc(&p->order_i, N));
+        // every order is scattered through (pos[order[p]] = p): ids in range from the start
+        if (n > 0) k_identity<<<grid_for(n, 256), 256>>>(n, p->order_i);
         TRYP(dalloc(&p->okey, N));
         TRYP(dalloc(&p->okey2, N));
         TRYP(dalloc(&p->ok32, N));

@@ -109,7 +109,8 @@ struct gs_plan {
     double* q2 = nullptr;
     double* q3 = nullptr;
     int* order = nullptr;                // topological order of the last flow sweep
-    int* order_i = nullptr;              // order of the snapshot (unfilled) flow graph
+    int* order_i = nullptr;              // order of the snapshot (unfilled) flow graph (the identity before the first)
+    int snap_tiles = 0;                  // that graph is tile records (TG_SNAP) and order_i was not sorted for it
     int order_i_valid = 0;
     int tie_m = 0;                       // vertices in surface tie groups of the last flow_order
     int pdir_bound = 0;                  // pdir + 1 <= pdir_bound after the last fill (0: unknown)

@@ -1131,7 +1131,11 @@ static int ordered_status(gs_plan* p, int* st) {
 
 // The tile dataflow (gs_tiles.cu) solves the FP64 sweeps of every plan whose
 // tiles fit; the ordered sweeps remain for larger meshes and for the FP32
-// sweeps of the precision form, and only they need an order.
+// sweeps of the precision form, and only they need an order.  The precision may
+// be set between two stages: what reads the snapshot graph of the last flow
+// accumulation (the flux, stream power, a cascade that merges its order) takes
+// the form that accumulation left (snap_tiles), FP64 tile sweeps where there is
+// no order.
 // On meshes whose records do not fit beside the values, the cascade's flow alone
 // is solved on tiles (tl_cas), with the records in L2: the sweep takes longer
 // than the ordered one (1,060 and 820 us at 2,621,442 vertices, 310 and 190 at
@@ -1140,6 +1144,8 @@ static int ordered_status(gs_plan* p, int* st) {
 // The snapshot graph's order is sorted beside the fill and serves other sweeps
 // too, and a recorded step keeps the orders for its adjoint.
 bool flow_needs_order(const gs_plan* p, int graph) {
+    if (graph == TG_FLUX || graph == TG_UP) return !p->snap_tiles;
+    if (graph == TG_CASCADE && p->snap_tiles) return false;
     if (p->fp32) return true;
     if (p->tl_nt > 0) return false;
     return !(graph == TG_CASCADE && p->tl_cas > 0 && !p->rec);
@@ -1223,7 +1229,7 @@ int spl_sweep(gs_plan* p, const int* rcv, const double* c, const int8_t* rslot, 
     if (n == 0) return GS_OK;
     const int ok = reuse_order && p->order_i_valid;
     if (!ok) return spl_sweep_counted(p, rcv, c, rslot, hold, s, cycle_nodes);
-    if (!flow_needs_order(p)) {
+    if (!flow_needs_order(p, TG_UP)) {
         // receivers first; every edge must be one of the checked snapshot
         // graph, else the sweep stops at once and the counter-based one runs
         GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));

@@ -110,6 +110,10 @@ int gs_plan_tune(gs_plan* plan, int32_t knob, int32_t value);
  * FP32) until max|r| <= tol max|b| (sweeps) or |r|_2 <= max(rtol, tol) |b|_2
  * (CG); receivers, pit filling, the cascade and every mass sum stay FP64.
  * bits = 64 (default): the plain FP64 path.
+ * It may be set at any time.  gs_erodep_spl and gs_sed_change solve over the
+ * graph of the last gs_flow_accumulation in the form that call left it: after
+ * one in FP64 on mesh tiles, which has no order for the FP32 sweeps, they run
+ * in FP64 until the next accumulation.
  */
 int gs_plan_set_precision(gs_plan* plan, int32_t bits, double tol);
 int gs_plan_tuning(const gs_plan* plan, int32_t knob);
