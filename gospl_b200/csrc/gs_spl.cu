@@ -394,7 +394,7 @@ static int coupled_ed(gs_plan* p, const double* hold, const double* fal, const u
     const int st = gmres_solve(p, op, a, x, 1.0e-13, 200, &applies, &relres);
     p->ed_iters = applies;
     p->ed_relres = relres;
-    if (p->tl_nt > 0) {
+    if (!flow_needs_order(p, TG_UP)) {
         // the sweeps were only queued: one that stopped explains a failure
         const int sw = tile_status(p, "transport-limited SPL: a sweep did not complete");
         if ((unsigned)sw == TILE_REJECTED) {

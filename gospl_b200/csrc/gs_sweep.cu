@@ -1547,8 +1547,9 @@ int spl_refine32(gs_plan* p, const int* rcv, const double* c, const double* hold
 // Plain FP64 sweeps with caller-given right-hand sides, for solvers that
 // apply the flow or SPL inverse repeatedly (the coupled erosion-deposition
 // system), after sweeps_prepare on the snapshot graph rcv/wgt/rslot and the
-// SPL coefficients c.  On tiles the sweeps are only queued: their status is
-// read at the end of the solver (tile_status).
+// SPL coefficients c, in the form the last flow accumulation left that graph
+// (an order after an FP32 one, whose sweeps here stay FP64).  On tiles the sweeps
+// are only queued: their status is read at the end of the solver (tile_status).
 static int build_donors(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot) {
     const int n = (int)p->n;
     GS_CUDA(cudaMemsetAsync(p->don_mask, 0, sizeof(uint32_t) * n, p->stream));
@@ -1561,7 +1562,7 @@ static int build_donors(gs_plan* p, const int* rcv, const double* wgt, const int
 
 int sweep_flow_rhs(gs_plan* p, const double* wgt, const int* order, const double* b, double* x) {
     const int n = (int)p->n;
-    if (p->tl_nt > 0) return tile_solve(p, TG_CASCADE, false, b, x, p->i_scalar + 14);
+    if (!flow_needs_order(p, TG_UP)) return tile_solve(p, TG_CASCADE, false, b, x, p->i_scalar + 14);
     GS_CUDA(cudaMemsetAsync(p->ctr, 0, sizeof(unsigned) * 8, p->stream));
     launch(p, k_fill_sent, grid_for(n, 256), 256, n, x);
     FlowOrd op{n, p->nbr, p->don_mask, p->don_k, p->sorder, wgt, b, x};
@@ -1578,7 +1579,7 @@ int sweep_flow_rhs(gs_plan* p, const double* wgt, const int* order, const double
 
 int sweep_spl_rhs(gs_plan* p, const int* rcv, const double* c, const int* order2, const double* rhs, double* x) {
     const int n = (int)p->n;
-    if (p->tl_nt > 0) return tile_solve(p, TG_UP, true, rhs, x, p->i_scalar + 14);
+    if (!flow_needs_order(p, TG_UP)) return tile_solve(p, TG_UP, true, rhs, x, p->i_scalar + 14);
     GS_CUDA(cudaMemsetAsync(p->ctr, 0, sizeof(unsigned) * 8, p->stream));
     launch(p, k_fill_sent, grid_for(n, 256), 256, n, x);
     SplOrd op{n, p->R, rcv, c, rhs, x};
@@ -1595,7 +1596,7 @@ int sweep_spl_rhs(gs_plan* p, const int* rcv, const double* c, const int* order2
 
 int sweeps_prepare(gs_plan* p, const int* rcv, const double* wgt, const int8_t* rslot, const double* c) {
     const int n = (int)p->n;
-    if (p->tl_nt > 0) {
+    if (!flow_needs_order(p, TG_UP)) {
         // edges outside the checked snapshot graph stop the sweeps (i_scalar[14])
         const uint16_t* ref = p->tl_graph[TG_SNAP].pm;
         GS_CUDA(cudaMemsetAsync(p->i_scalar + 14, 0, sizeof(int), p->stream));
