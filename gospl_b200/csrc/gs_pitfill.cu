@@ -1059,7 +1059,7 @@ __global__ void __launch_bounds__(256) k_relax_active(const int* __restrict__ m_
 // the distances that shorten through them until none does: the fixed point of
 // all edges, which is the search over all depressions.  A depression whose
 // visited set does not fit shared memory (FLAT_MAX cells) makes that search run
-// instead.
+// instead, and so does a mesh with edges that only one of their ends lists.
 constexpr int FLAT_MAX = 1 << 20;   // 128 KB of visited bits
 constexpr int FLAT_CAP = 4096;      // frontier entries in shared memory; the rest in global memory
 enum { FL_BIG = 0, FL_MID = 1, FL_TICKET = 2, FL_RIM = 3, FL_ALL = 4, FL_DEPTH = 5, FL_NCTL = 8 };
@@ -1970,8 +1970,11 @@ int fill_elevation(gs_plan* p, const double* h, double sealevel, double ofill, d
     // on the main stream: they share only read-only inputs, and the sea reset
     // of lFill in k_flat_dirs touches open-sea cells, which hold no pit.
     p->pdir_bound = 0;
-    // GS_TUNE_FLAT_BFS > 0 asks for the search over all depressions in tiles
-    const bool all_at_once = p->bfs_window > 0;
+    // GS_TUNE_FLAT_BFS > 0 asks for the search over all depressions in tiles.
+    // An edge that only one of its ends lists is walked from that end alone: the
+    // search over all depressions follows the list of the cell it has reached,
+    // the one by depression looks into the lists of the cells it has not.
+    const bool all_at_once = p->bfs_window > 0 || !p->mutual;
     int last[2] = {0, 0};
     if (all_at_once) {
         GS_TRY(flat_compact(p, pit_ids));
