@@ -540,6 +540,7 @@ __global__ void k_bfs_local_scatter(int M, const int* __restrict__ l2g, const in
 }
 
 constexpr int LBFS_CAP = 6144;
+constexpr int LBFS_SMEM = 200 * 1024;   // frontiers and visited set; larger sets are searched in tiles
 
 // S4: int4 words of a packed adjacency row (S = 4 * S4 ints, row[0] the
 // count).  A level's cost is the instruction chain of its busiest warp, so
@@ -663,6 +664,7 @@ __global__ void __launch_bounds__(1024) k_bfs_local(int M, int S, const int* __r
 // only decrease and a window is closed only when no cell of it is pending, so
 // every distance is the breadth-first hop count (exact, no timed wait).
 constexpr int BFT_THREADS = 512;
+constexpr int BFT_SMEM = 112 * 1024;   // most of a block's shared memory
 
 __global__ void __launch_bounds__(BFT_THREADS, 2) k_bfs_tiles(int M, int S, int T, const int* __restrict__ rows,
                                                               const int* __restrict__ seeds,
@@ -1618,9 +1620,8 @@ static int launch_coop(gs_plan* p, const void* fn, int blocks, int threads, void
 // as stay co-resident.
 static int bfs_tiles(gs_plan* p, int M, int S, const int* rows, int* ld) {
     int T = 4096;
-    while (T > 256 && (size_t)T * (S + 5) * sizeof(int) > 112 * 1024) T >>= 1;
+    while (T > 256 && (size_t)T * (S + 5) * sizeof(int) > BFT_SMEM) T >>= 1;
     const size_t smem = (size_t)T * (S + 5) * sizeof(int);
-    GS_CUDA(cudaFuncSetAttribute(k_bfs_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int occ = 0;
     GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bfs_tiles, BFT_THREADS, smem));
     if (occ < 1) {
@@ -1723,12 +1724,11 @@ static int flat_search_all(gs_plan* p, int M, const double* lfill, const int* pi
            p->i_scalar + 6);
     GS_LAUNCH();
     const size_t smem1 = sizeof(unsigned) * (size_t)((M + 31) / 32) + sizeof(int) * 2 * LBFS_CAP;
-    if (p->bfs_window > 0 || smem1 > 200 * 1024) {
+    if (p->bfs_window > 0 || smem1 > LBFS_SMEM) {
         GS_TRY(bfs_tiles(p, M, S, rows, ldv));
     } else {
         // one block: visited bitmap and frontiers in shared memory
         auto run = [&](auto kern) -> int {
-            GS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
             cudaEvent_t stop = nullptr;
             if (p->profiling) prof_begin(p, (const void*)kern, &stop);
             kern<<<1, 1024, smem1, p->stream>>>(M, S, (const int*)rows, (const int*)p->front0, p->i_scalar + 6,
@@ -1795,7 +1795,6 @@ static int flat_search_pits(gs_plan* p, int m, const FlatArgs& a) {
         const bool wide = m > 32768;
         const int T = wide ? 1024 : 512, smem = (std::min(m, FLAT_MAX) + 31) / 32 * 4;
         auto kern = wide ? k_flat_big<G, 1024> : k_flat_big<G, 512>;
-        GS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         cudaEvent_t stop = nullptr;
         if (p->profiling) prof_begin(p, (const void*)kern, &stop);
         kern<<<std::min(p->sm_count * 2, np1), T, smem, p->stream>>>(
@@ -1813,6 +1812,30 @@ static int flat_search_pits(gs_plan* p, int m, const FlatArgs& a) {
     GS_TRY(flat_dirs_launch(p, a, ctl + FL_ALL, ctl + FL_DEPTH));
     GS_CUDA(cudaMemcpyAsync(p->h_pinned + 2, ctl + FL_DEPTH, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
     GS_CUDA(cudaMemcpyAsync(p->h_pinned + 3, ctl + FL_ALL, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+    return GS_OK;
+}
+
+// The shared memory that the flat searches of a mesh of W slots may ask for.  The
+// limit belongs to the kernel and the device, not to the plan, and plans of other
+// threads launch meanwhile: it is set once per plan, always to the same value,
+// and never lowered to what one launch needs.
+int flat_limits(int W) {
+    const auto limit = [](auto kern, int bytes) {
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    const int S4 = (W + 1 + 3) / 4, seen = FLAT_MAX / 8;
+    GS_CUDA(limit(k_bfs_tiles, BFT_SMEM));
+    if (S4 <= 1) GS_CUDA(limit(k_bfs_local<1>, LBFS_SMEM));
+    else if (S4 == 2) GS_CUDA(limit(k_bfs_local<2>, LBFS_SMEM));
+    else if (S4 == 3) GS_CUDA(limit(k_bfs_local<3>, LBFS_SMEM));
+    else GS_CUDA(limit(k_bfs_local<4>, LBFS_SMEM));
+    if (W <= 8) {
+        GS_CUDA(limit(k_flat_big<8, 512>, seen));
+        GS_CUDA(limit(k_flat_big<8, 1024>, seen));
+    } else {
+        GS_CUDA(limit(k_flat_big<16, 512>, seen));
+        GS_CUDA(limit(k_flat_big<16, 1024>, seen));
+    }
     return GS_OK;
 }
 

@@ -310,6 +310,8 @@ int plan_create(int64_t nb, const int32_t* nnb, const int32_t* ngb, const double
             goto fail;
         }
     }
+    st = flat_limits(W);
+    if (st != GS_OK) goto fail;
     p->mutual = mutual;
     st = mutual ? tiles_setup(p, nnb, ngb) : GS_OK;
     if (st != GS_OK) goto fail;

@@ -397,6 +397,7 @@ int output_fields(gs_plan* p, const double* h, const double* cum_ed, const doubl
 
 void prof_begin(gs_plan* p, const void* fn, cudaEvent_t* stop);
 int coop_occupancy(int* per_sm);
+int flat_limits(int W);   // shared-memory limits of the flat searches, on the current device
 __global__ void k_cg_coop32(int n, int ng, const int* __restrict__ nbr, const int8_t* __restrict__ nnb,
                             const double* __restrict__ coef, const double* __restrict__ farea,
                             const uint8_t* __restrict__ fix, const double* __restrict__ rhs, float* x, float* r,

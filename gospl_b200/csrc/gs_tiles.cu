@@ -875,7 +875,9 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
         for (int div = 0; div < (cas ? 1 : 2) && ok; div++) {
             const void* k = sweep_kernel<NP>(div != 0, p->tl_keep);
             int o = 0;
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->tl_smem) != cudaSuccess ||
+            // (the limit is the kernel's, not the plan's: the device's own for every
+            // plan, so that no thread lowers it under another's launch)
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess ||
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, TS_THREADS, p->tl_smem) != cudaSuccess || o < 1)
                 ok = 0;
         }
@@ -1023,7 +1025,6 @@ int tile_solve(gs_plan* p, int which, bool div, const double* b, double* x, cons
         constexpr int NP = decltype(w)::value;
         const void* fn = sweep_kernel<NP>(div, p->tl_keep);
         void* args[] = {(void*)&a};
-        GS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->tl_smem));
         cudaEvent_t stop = nullptr;
         if (p->profiling) prof_begin(p, fn, &stop);
         // the blocks wait on one another: a cooperative launch keeps them all resident
