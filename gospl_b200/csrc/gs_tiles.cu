@@ -242,7 +242,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_tile_sweep(SweepArgs a) {
     };
     // absent successors count down a word of their lane that nothing reads
     const unsigned none = (unsigned)(nw + lane) * (KEEP == 0 ? 4u : 1u);
+    // The values that l's other predecessors released with their counts reach the
+    // taker through this thread, which saw the last count: a fence between that
+    // count and the queue entry (the taker's own stands behind its read of the entry)
     auto push = [&](unsigned l) {
+        fence_cta();
         const unsigned pos = atomicAdd(&s_tail, 1u);   // a vertex is pushed at most once: pos < T
         vq[pos] = (unsigned short)l;
     };
