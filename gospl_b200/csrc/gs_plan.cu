@@ -130,7 +130,7 @@ int plan_create(int64_t nb, const int32_t* nnb, const int32_t* ngb, const double
             h_vd[(size_t)s * n + i] = vdist[(size_t)i * 12 + s];
         }
     }
-    bool mutual = true;   // every edge is listed by both of its ends
+    bool mutual = true;   // every edge is listed by both of its ends, and once
     for (int i = 0; i < n; i++) {
         int slots[12], ids[12], cnt = 0;
         for (int s = 0; s < nnb[i]; s++) {
@@ -141,6 +141,7 @@ int plan_create(int64_t nb, const int32_t* nnb, const int32_t* ngb, const double
                 ids[at] = ids[at - 1];
                 slots[at] = slots[at - 1];
             }
+            if (at > 0 && ids[at - 1] == j) mutual = false;
             ids[at] = j;
             slots[at] = s;
             const int32_t* row = ngb + (size_t)j * 12;

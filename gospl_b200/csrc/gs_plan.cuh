@@ -125,7 +125,7 @@ struct gs_plan {
     double* c = nullptr;                 // SPL coefficients [R][n]
 
     // mesh tiles of the dataflow sweeps (gs_tiles.cu); tl_nt = 0: ordered sweeps
-    bool mutual = true;                  // every edge is listed by both of its ends
+    bool mutual = true;                  // every edge is listed by both of its ends, and once
     int tl_nt = 0;                       // tiles, one resident block each
     int tl_cas = 0;                      // tiles that only TG_CASCADE is solved on (tl_nt = 0)
     int tl_T = 0;                        // vertices per tile

@@ -803,7 +803,8 @@ static void grow_tiles(int n, const int32_t* nnb, const int32_t* ngb, int T, std
 // and a queue slot per vertex fit for 2.7 million vertices.
 // Not called for a mesh with an edge that only one of its ends lists (a vertex
 // of more than twelve neighbours, of which the reference keeps the first
-// twelve): solved vertices are announced through the neighbour lists.
+// twelve), nor where a vertex lists a neighbour twice: solved vertices are
+// announced through the neighbour lists, once per edge.
 int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
     const int n = (int)p->n;
     p->tl_nt = 0;
