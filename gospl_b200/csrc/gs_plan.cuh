@@ -133,6 +133,7 @@ struct gs_plan {
     int tl_cap = 0;                      // most cut edges of a tile
     int tl_par = 0;                      // half of tl_xb the next solve publishes in
     int tl_dirty = 0;                    // tl_xb and the status word need a reset
+    int tl_open = 0;                     // solves queued whose status nobody has read yet
     size_t tl_smem = 0;
     char* tl_pool = nullptr;             // the allocation that holds all of the following
     int* tl_perm = nullptr;              // tile-major position -> vertex (null: identity)

@@ -946,6 +946,11 @@ void tiles_free(gs_plan* p) {
 }
 
 static BuildArgs build_args(gs_plan* p, const TileGraph& g) {
+    // solves that a call queued and did not see the end of (it stopped on an
+    // error, or its stream was capturing and nothing ran) left the halves of
+    // tl_xb in a state that is not known
+    if (p->tl_open) p->tl_dirty = 1;
+    p->tl_open = 0;
     BuildArgs a = {};
     a.n = (int)p->n;
     a.T = p->tl_T;
@@ -1026,6 +1031,7 @@ int tile_solve(gs_plan* p, int which, bool div, const double* b, double* x, cons
     a.skip = skip;
     a.budget_ns = p->sweep_budget_ns;
     p->tl_par = 1 - p->tl_par;
+    p->tl_open = 1;
     return by_width(p, [&](auto w) -> int {
         constexpr int NP = decltype(w)::value;
         const void* fn = sweep_kernel<NP>(div, p->tl_keep);
@@ -1046,6 +1052,7 @@ int tile_status_async(gs_plan* p, int* host) {
 }
 
 int tile_status_check(gs_plan* p, int st, const char* what) {
+    p->tl_open = 0;
     if (st == 0) return GS_OK;
     p->tl_dirty = 1;   // values of the stopped solve are published: reset before the next
     if ((unsigned)st != TILE_REJECTED) set_error(st, what);
