@@ -29,7 +29,6 @@
 // bounded by the plan's sweep budget (GS_ETIMEOUT).
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <vector>
 
 #include "gs_plan.cuh"
@@ -729,60 +728,120 @@ const void* sweep_kernel(bool div, int keep) {
 
 }  // namespace
 
-// cut edges of each tile for the positions loc (null: identity)
-static void count_cuts(int n, const int32_t* nnb, const int32_t* ngb, int T, int nt, const int* loc,
-                       std::vector<int>& cuts) {
-    cuts.assign(nt, 0);
-    for (int i = 0; i < n; i++) {
-        const int ti = (loc ? loc[i] : i) / T;
-        for (int s = 0; s < nnb[i]; s++) {
-            const int j = ngb[(size_t)i * 12 + s];
-            if (j >= 0 && j < n && (loc ? loc[j] : j) / T != ti) cuts[ti]++;
+// Cut edges of a tile (one block): their number, or with FILL their tables from
+// c0[tile] on, by position and slot.  On the device, which has the neighbour rows
+// already: two passes on the host and the upload of the tables took 12 ms of a
+// plan's creation at 160,000 vertices and 30 at 655,000.
+constexpr int CUT_THREADS = 256;
+template <bool FILL>
+__global__ void __launch_bounds__(CUT_THREADS) k_cuts(int n, int T, const int* __restrict__ perm,
+                                                      const int* __restrict__ loc, const int* __restrict__ nbr,
+                                                      const int8_t* __restrict__ nnb, int* count,
+                                                      const int* __restrict__ c0, unsigned* cut_q, unsigned* cut_l,
+                                                      uint16_t* cut_idx) {
+    constexpr int NW = CUT_THREADS / 32;
+    __shared__ int s_warp[NW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
+    const int p0 = tile * T, m = min(T, n - p0);
+    int run = 0;
+    for (int base = 0; base < m; base += CUT_THREADS) {
+        const int p = p0 + base + tid;
+        int cnt = 0, i = 0;
+        unsigned cut = 0u;
+        if (base + tid < m) {
+            i = perm ? perm[p] : p;
+            const int deg = nnb[i];
+            for (int s = 0; s < deg; s++) {
+                const int j = nbr[(size_t)s * n + i];
+                if (j >= 0 && j < n && (loc ? loc[j] : j) / T != tile) cut |= 1u << s;
+            }
+            cnt = __popc(cut);
         }
+        int incl = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        __syncthreads();   // the sums of the batch before are read
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < NW; w++) {
+            if (w < warp) before += s_warp[w];
+            all += s_warp[w];
+        }
+        if (FILL) {
+            int at = run + before + incl - cnt;
+            for (; cut; cut &= cut - 1u, at++) {
+                const int s = __ffs(cut) - 1, j = nbr[(size_t)s * n + i];
+                cut_idx[(size_t)s * n + p] = (uint16_t)at;
+                cut_q[c0[tile] + at] = (unsigned)(loc ? loc[j] : j);
+                cut_l[c0[tile] + at] = (unsigned)(p - p0) | ((unsigned)s << 16);
+            }
+        }
+        run += all;
     }
+    if (!FILL && tid == 0) count[tile] = run;
+}
+
+__global__ void k_loc(int n, const int* __restrict__ perm, int* loc) {
+    int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n) loc[perm[p]] = p;
+}
+
+// cut edges of each tile for the positions loc (null: identity); scratch: scanbuf
+static int count_cuts(gs_plan* p, int T, int nt, const int* perm, const int* loc, std::vector<int>& cuts) {
+    cuts.resize(nt);
+    k_cuts<false><<<nt, CUT_THREADS>>>((int)p->n, T, perm, loc, p->nbr, p->nnb, p->scanbuf, nullptr, nullptr, nullptr,
+                                       nullptr);
+    GS_LAUNCH();
+    GS_CUDA(cudaMemcpy(cuts.data(), p->scanbuf, sizeof(int) * nt, cudaMemcpyDeviceToHost));
+    return GS_OK;
 }
 
 // Tile-major order of the vertices by growing one tile after the other
-// breadth-first from an unassigned vertex next to the tiles already grown.
-static void grow_tiles(int n, const int32_t* nnb, const int32_t* ngb, int T, std::vector<int>& perm) {
-    perm.clear();
-    perm.reserve(n);
-    std::vector<char> done(n, 0);
-    std::vector<int> mark(n, -1), front, rest;
+// breadth-first from an unassigned vertex next to the tiles already grown; by
+// id within a tile, so that neighbours in memory stay together.
+static void grow_tiles(int n, const int32_t* nnb, const int32_t* ngb, int T, int nt, std::vector<int>& perm) {
+    std::vector<int> tile_of(n, -1), mark(n, -1), front, rest;
     size_t rh = 0;
-    int scan = 0;
-    for (int tile = 0; (int)perm.size() < n; tile++) {
+    int scan = 0, done = 0;
+    for (int tile = 0; done < n; tile++) {
         front.clear();
         size_t h = 0;
-        for (int cnt = 0; cnt < T && (int)perm.size() < n;) {
+        for (int cnt = 0; cnt < T && done < n;) {
             if (h == front.size()) {
                 int seed = -1;
                 while (rh < rest.size() && seed < 0) {
                     const int c = rest[rh++];
-                    if (!done[c]) seed = c;
+                    if (tile_of[c] < 0) seed = c;
                 }
                 if (seed < 0) {
-                    while (done[scan]) scan++;
+                    while (tile_of[scan] >= 0) scan++;
                     seed = scan;
                 }
                 mark[seed] = tile;
                 front.push_back(seed);
             }
             const int v = front[h++];
-            if (done[v]) continue;
-            done[v] = 1;
-            perm.push_back(v);
+            if (tile_of[v] >= 0) continue;
+            tile_of[v] = tile;
+            done++;
             cnt++;
             for (int s = 0; s < nnb[v]; s++) {
                 const int j = ngb[(size_t)v * 12 + s];
-                if (j < 0 || j >= n || done[j] || mark[j] == tile) continue;
+                if (j < 0 || j >= n || tile_of[j] >= 0 || mark[j] == tile) continue;
                 mark[j] = tile;
                 front.push_back(j);
             }
         }
         for (; h < front.size(); h++)
-            if (!done[front[h]]) rest.push_back(front[h]);
+            if (tile_of[front[h]] < 0) rest.push_back(front[h]);
     }
+    std::vector<int> at(nt);
+    for (int t = 0; t < nt; t++) at[t] = t * T;   // every tile but the last is full
+    perm.resize(n);
+    for (int v = 0; v < n; v++) perm[at[tile_of[v]]++] = v;
 }
 
 // The plan's tiles: one per SM but SM_SPARE (a cooperative launch waits for
@@ -791,7 +850,8 @@ static void grow_tiles(int n, const int32_t* nnb, const int32_t* ngb, int T, std
 // and 160,000 vertices).  Consecutive ids are kept as they are when their tiles
 // cut at most twice the edges of grown ones (meshes numbered along a
 // space-filling curve: values then stay in vertex order); other numberings
-// (rows of a lattice, mesh generators) get grown tiles.
+// (rows of a lattice, mesh generators) get grown tiles (3 ms on the host at
+// 160,000 vertices).
 // A tile must fit its block's shared memory with the hot part of its records
 // (about 3,200 vertices a tile, 460,000 in all).  Larger meshes keep the
 // ordered sweeps (tl_nt = 0) but for the cascade's flow (tl_cas), which would
@@ -820,53 +880,41 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
     const int T = (int)T64;
     const bool cas = tile_smem(T, 0, HOT + 8) > room;   // the cascade's flow alone
     const int nt = (n + T - 1) / T;
-    std::vector<int> perm, loc, cuts, gcuts;
-    count_cuts(n, nnb, ngb, T, nt, nullptr, cuts);
+    std::vector<int> cuts, gcuts;
+    const int* d_perm = nullptr;   // tile-major order, in scratch until the pool is there
+    const int* d_loc = nullptr;
+    GS_TRY(count_cuts(p, T, nt, nullptr, nullptr, cuts));
+    int64_t total = 0;
+    for (int c : cuts) total += c;
+    const double side = sqrt((double)T) * nt;
     if (cas) {
         // consecutive ids as they are, or not at all: growing tiles of so many
         // vertices costs the host more than many steps save.  A compact patch cuts
         // about 8 sqrt(T) edges, one along a space-filling curve up to twice that,
         // the strips of a lattice's rows some 60 sqrt(T).
-        int64_t total = 0;
-        for (int c : cuts) total += c;
-        if ((double)total > 24.0 * sqrt((double)T) * nt) return GS_OK;
-    } else if (nt > 1) {
-        grow_tiles(n, nnb, ngb, T, perm);
-        // by id within a tile: neighbours in memory stay together
-        for (int t = 0; t < nt; t++)
-            std::sort(perm.begin() + (size_t)t * T, perm.begin() + std::min<size_t>(n, (size_t)(t + 1) * T));
-        loc.resize(n);
-        for (int q = 0; q < n; q++) loc[perm[q]] = q;
-        count_cuts(n, nnb, ngb, T, nt, loc.data(), gcuts);
-        int64_t a = 0, b = 0;
-        for (int t = 0; t < nt; t++) {
-            a += cuts[t];
-            b += gcuts[t];
+        if ((double)total > 24.0 * side) return GS_OK;
+    } else if (nt > 1 && !(T > TILE_MIN && (double)total <= 16.0 * side)) {
+        // (a curve's tiles are kept without growing others where that costs
+        // milliseconds, 6 at 164,000 vertices; grown ones cut 8.0 to 8.4 sqrt(T))
+        std::vector<int> perm;
+        grow_tiles(n, nnb, ngb, T, nt, perm);
+        GS_CUDA(cudaMemcpy(p->comp, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+        k_loc<<<grid_for(n, 256), 256>>>(n, p->comp, p->lab);
+        GS_LAUNCH();
+        GS_TRY(count_cuts(p, T, nt, p->comp, p->lab, gcuts));
+        int64_t grown = 0;
+        for (int c : gcuts) grown += c;
+        if (total > 2 * grown) {
+            cuts.swap(gcuts);
+            d_perm = p->comp;
+            d_loc = p->lab;
         }
-        if (a <= 2 * b) perm.clear();
-        else cuts.swap(gcuts);
     }
-    const int* lp = perm.empty() ? nullptr : loc.data();
     const int cap = std::max(1, *std::max_element(cuts.begin(), cuts.end()));
     // (64 groups of the pollers' cut edges, 16-bit value indices)
     if (cap > 64 * POLL_LANES * POLL_EDGES || T + cap > 0xffff) return GS_OK;
-    std::vector<int> c0(nt + 1, 0), at(nt);
+    std::vector<int> c0(nt + 1, 0);
     for (int t = 0; t < nt; t++) c0[t + 1] = c0[t] + cuts[t];
-    for (int t = 0; t < nt; t++) at[t] = c0[t];
-    std::vector<unsigned> cq(std::max(c0[nt], 1)), cl(std::max(c0[nt], 1));
-    std::vector<uint16_t> ci((size_t)p->W * n, 0);
-    for (int q = 0; q < n; q++) {
-        const int i = lp ? perm[q] : q, t = q / T;
-        for (int s = 0; s < nnb[i]; s++) {
-            const int j = ngb[(size_t)i * 12 + s];
-            if (j < 0 || j >= n) continue;
-            const int qj = lp ? loc[j] : j;
-            if (qj / T == t) continue;
-            ci[(size_t)s * n + q] = (uint16_t)(at[t] - c0[t]);
-            cq[at[t]] = (unsigned)qj;
-            cl[at[t]++] = (unsigned)(q - t * T) | ((unsigned)s << 16);
-        }
-    }
     p->tl_T = T;
     p->tl_cap = cap;
     p->tl_np = p->W <= 6 ? 6 : p->W <= 8 ? 8 : 12;
@@ -890,27 +938,25 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
     });
     cudaGetLastError();
     if (!ok) return GS_OK;
-    // one allocation: the tile tables (one upload), the published values, the
-    // status word and the records of the three graphs
-    const size_t N = (size_t)n;
+    // one allocation: the tile tables, the published values, the status word and
+    // the records of the three graphs
+    const size_t N = (size_t)n, ncut = (size_t)std::max(c0[nt], 1);
     size_t rec_bytes = 0;
     by_width(p, [&](auto w) -> int {
         rec_bytes = N * Rec<decltype(w)::value>::BYTES;
         return GS_OK;
     });
-    std::vector<char> host;
-    auto put = [&](const void* src, size_t bytes) {
-        const size_t at = host.size();
-        host.resize(at + (bytes + 31) / 32 * 32);
-        if (bytes) memcpy(host.data() + at, src, bytes);
+    size_t pool = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = pool;
+        pool += (bytes + 31) / 32 * 32;
         return at;
     };
-    const unsigned zero = 0u;
-    const size_t o_status = put(&zero, sizeof(zero)), o_c0 = put(c0.data(), sizeof(int) * c0.size()),
-                 o_cq = put(cq.data(), sizeof(unsigned) * cq.size()), o_cl = put(cl.data(), sizeof(unsigned) * cl.size()),
-                 o_ci = put(ci.data(), sizeof(uint16_t) * ci.size()),
-                 o_pm = put(perm.data(), lp ? sizeof(int) * N : 0), o_lc = put(loc.data(), lp ? sizeof(int) * N : 0);
-    const size_t o_xb = host.size(), o_g = o_xb + (2 * N * sizeof(double) + 31) / 32 * 32;
+    const size_t ids = d_perm ? sizeof(int) * N : 0;
+    const size_t o_status = take(sizeof(unsigned)), o_c0 = take(sizeof(int) * c0.size()),
+                 o_cq = take(sizeof(unsigned) * ncut), o_cl = take(sizeof(unsigned) * ncut),
+                 o_ci = take(sizeof(uint16_t) * p->W * N), o_pm = take(ids), o_lc = take(ids),
+                 o_xb = take(2 * N * sizeof(double)), o_g = pool;
     const size_t g_bytes = rec_bytes + (N * sizeof(uint16_t) + 31) / 32 * 32;
     cudaError_t e = cudaMalloc((void**)&p->tl_pool, o_g + (cas ? 1 : TG_N) * g_bytes);
     if (e != cudaSuccess) {
@@ -919,15 +965,24 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
         set_error(GS_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         return GS_ENOMEM;
     }
-    GS_CUDA(cudaMemcpy(p->tl_pool, host.data(), host.size(), cudaMemcpyHostToDevice));
     p->tl_status = (unsigned*)(p->tl_pool + o_status);
     p->tl_cut0 = (int*)(p->tl_pool + o_c0);
     p->tl_cut_q = (unsigned*)(p->tl_pool + o_cq);
     p->tl_cut_l = (unsigned*)(p->tl_pool + o_cl);
     p->tl_cut_idx = (uint16_t*)(p->tl_pool + o_ci);
-    p->tl_perm = lp ? (int*)(p->tl_pool + o_pm) : nullptr;
-    p->tl_loc = lp ? (int*)(p->tl_pool + o_lc) : nullptr;
+    p->tl_perm = d_perm ? (int*)(p->tl_pool + o_pm) : nullptr;
+    p->tl_loc = d_perm ? (int*)(p->tl_pool + o_lc) : nullptr;
     p->tl_xb = (double*)(p->tl_pool + o_xb);
+    GS_CUDA(cudaMemset(p->tl_status, 0, sizeof(unsigned)));
+    GS_CUDA(cudaMemcpy(p->tl_cut0, c0.data(), sizeof(int) * c0.size(), cudaMemcpyHostToDevice));
+    if (d_perm) {
+        GS_CUDA(cudaMemcpy(p->tl_perm, d_perm, ids, cudaMemcpyDeviceToDevice));
+        GS_CUDA(cudaMemcpy(p->tl_loc, d_loc, ids, cudaMemcpyDeviceToDevice));
+    }
+    k_cuts<true><<<nt, CUT_THREADS>>>(n, T, p->tl_perm, p->tl_loc, p->nbr, p->nnb, nullptr, p->tl_cut0, p->tl_cut_q,
+                                      p->tl_cut_l, p->tl_cut_idx);
+    GS_LAUNCH();
+    GS_CUDA(cudaDeviceSynchronize());
     for (int g = 0; g < TG_N; g++) {
         if (cas && g != TG_CASCADE) continue;
         p->tl_graph[g].rec = p->tl_pool + o_g + (cas ? 0 : g) * g_bytes;
