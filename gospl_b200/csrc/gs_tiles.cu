@@ -958,12 +958,10 @@ int tiles_setup(gs_plan* p, const int32_t* nnb, const int32_t* ngb) {
                  o_ci = take(sizeof(uint16_t) * p->W * N), o_pm = take(ids), o_lc = take(ids),
                  o_xb = take(2 * N * sizeof(double)), o_g = pool;
     const size_t g_bytes = rec_bytes + (N * sizeof(uint16_t) + 31) / 32 * 32;
-    cudaError_t e = cudaMalloc((void**)&p->tl_pool, o_g + (cas ? 1 : TG_N) * g_bytes);
-    if (e != cudaSuccess) {
+    if (cudaMalloc((void**)&p->tl_pool, o_g + (cas ? 1 : TG_N) * g_bytes) != cudaSuccess) {
         p->tl_pool = nullptr;
         cudaGetLastError();
-        set_error(GS_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        return GS_ENOMEM;
+        return GS_OK;   // no room for the records: the ordered sweeps need none
     }
     p->tl_status = (unsigned*)(p->tl_pool + o_status);
     p->tl_cut0 = (int*)(p->tl_pool + o_c0);
