@@ -232,9 +232,10 @@ __device__ __forceinline__ double mfd_slope(double d, double l, double fexp, boo
 // and nothing has to be ranked.  The powers of the land vertices bound it, then
 // the stores: eight directions of 655,362 vertices and their masks take 56 us,
 // where the general form (arrays in local memory) and a pass for the masks took
-// 73.  Six slots: 64 registers for eight blocks an SM, 4 % faster than 78.
-template <int NP>
-__global__ void __launch_bounds__(128, NP == 6 ? 8 : 1) k_mfd_all(int n, int R, double expo, const double* __restrict__ elev,
+// 73.  Six slots: 64 registers for eight blocks an SM, 4 % faster than 78.  MINB,
+// the blocks an SM that the registers have to allow: see two_waves.
+template <int NP, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_mfd_all(int n, int R, double expo, const double* __restrict__ elev,
                                                   double sl, const int* __restrict__ gid, const int* __restrict__ nbr,
                                                   const double* __restrict__ elen, const int8_t* __restrict__ nnb,
                                                   int* __restrict__ rcv, double* __restrict__ dist,
@@ -295,8 +296,10 @@ __global__ void __launch_bounds__(128, NP == 6 ? 8 : 1) k_mfd_all(int n, int R, 
 // numbering (one partition).  The gathers of a vertex are in flight together: in
 // a loop over its slots, and once more in the second pass over them, three
 // directions took 22 us on 20,000 vertices and 125 on 2.6 million, now 18 and 112.
+// NP = 0 is that loop: 64 registers whatever the slots, for the meshes that
+// two_waves sends here.
 template <int RM, int NP>
-__global__ void __launch_bounds__(128, NP == 6 ? 8 : 1) k_mfd_receivers_r(int n, double expo, const double* __restrict__ elev,
+__global__ void __launch_bounds__(128, NP == 6 || NP == 0 ? 8 : 1) k_mfd_receivers_r(int n, double expo, const double* __restrict__ elev,
                                                           double sl, const int* __restrict__ gid,
                                                           const int* __restrict__ nbr, const double* __restrict__ elen,
                                                           const int8_t* __restrict__ nnb, int* __restrict__ rcv,
@@ -316,9 +319,22 @@ __global__ void __launch_bounds__(128, NP == 6 ? 8 : 1) k_mfd_receivers_r(int n,
         dir_masks(post, k, sl, true);
         return;
     }
-    int c[NP];
-    double l[NP], d[NP], fexp;
-    mfd_gather<NP>(k, n, hk, elev, nbr, elen, nnb, expo, c, l, d, fexp);
+    const int deg = nnb[k];
+    constexpr int NG = NP ? NP : 1;
+    int c[NG];
+    double l[NG], d[NG], fexp;
+    if constexpr (NP != 0) mfd_gather<NP>(k, n, hk, elev, nbr, elen, nnb, expo, c, l, d, fexp);
+    else {
+        double e = 0.0;
+        for (int s = 0; s < deg; s++) {
+            const int j = nbr[(size_t)s * n + k];
+            const double ls = elen[(size_t)s * n + k];
+            if (j < 0 || !(ls > 0.0)) continue;
+            const double g = (hk - elev[j]) / ls;
+            e = (g > e) ? g : e;
+        }
+        fexp = e > 0 ? 5.0 * ((e < 1.0) ? e : 1.0) + expo : 1.0;
+    }
     const bool fexp_int = (fexp == floor(fexp));
     // candidates: slope (scaled by the global-id tie-break), kept descending;
     // strict > keeps the earlier slot ahead of an equal value
@@ -334,30 +350,39 @@ __global__ void __launch_bounds__(128, NP == 6 ? 8 : 1) k_mfd_receivers_r(int n,
     int kk = 0;
     double tot_all = 0.0;
     bool tie = false;
-#pragma unroll
-    for (int s = 0; s < NP; s++) {
-        if (c[s] < 0) continue;
-        const double val = mfd_slope(d[s], l[s], fexp, fexp_int);
-        if (!(val > 0.0)) continue;
-        double x = val * (1.0 - 1.0e-15 * (double)(gid ? gid[c[s]] : c[s]));
+    auto take = [&](int s, int j, double ls, double ds) {
+        const double val = mfd_slope(ds, ls, fexp, fexp_int);
+        if (!(val > 0.0)) return;
+        double x = val * (1.0 - 1.0e-15 * (double)(gid ? gid[j] : j));
         mask |= 1u << s;
         kk++;
         tot_all = tot_all + x;
-        int xs = s, xi = c[s];
+        int xs = s, xi = j;
 #pragma unroll
-        for (int j = 0; j <= RM; j++) tie |= (x == tv[j]);
+        for (int q = 0; q <= RM; q++) tie |= (x == tv[q]);
 #pragma unroll
-        for (int j = 0; j <= RM; j++) {
-            if (x > tv[j]) {
-                const double t = tv[j];
-                const int a = ts[j], b = tid[j];
-                tv[j] = x;
-                ts[j] = xs;
-                tid[j] = xi;
+        for (int q = 0; q <= RM; q++) {
+            if (x > tv[q]) {
+                const double t = tv[q];
+                const int a = ts[q], b = tid[q];
+                tv[q] = x;
+                ts[q] = xs;
+                tid[q] = xi;
                 x = t;
                 xs = a;
                 xi = b;
             }
+        }
+    };
+    if constexpr (NP != 0) {
+#pragma unroll
+        for (int s = 0; s < NP; s++)
+            if (c[s] >= 0) take(s, c[s], l[s], d[s]);
+    } else {
+        for (int s = 0; s < deg; s++) {
+            const int j = nbr[(size_t)s * n + k];
+            const double ls = elen[(size_t)s * n + k];
+            if (j >= 0 && ls > 0.0) take(s, j, ls, hk - elev[j]);
         }
     }
     double sw = 0.0;
@@ -485,6 +510,17 @@ int sink_mask(gs_plan* p, const double* wgt, const uint8_t* sea, uint8_t* lsink)
     return GS_OK;
 }
 
+// More vertices than two waves of a form with `blocks` blocks of 128 an SM.  With
+// up to two, the unrolled forms gain from their gathers in flight; with more, the
+// blocks of 94 to 118 registers for 8 or 12 slots (and the spills of four
+// directions at 6) cost more than that gives, and 64 registers are faster.  B200,
+// us for the receivers and masks, lattices of 8 slots, unrolled and 64 registers:
+// three directions 14 and 18 at 20,000 vertices, 33.0 and 34.3 at 160,000, 73 and 65
+// at 400,000, 170 and 140 at 900,000; four 14 and 18, 41 and 37, 84 and 70, 209 and
+// 151; eight (all kept) 15.4 and 16.5, 43 and 37, 96 and 80, 194 and 163.  Spheres,
+// four directions: 30.5 and 30.2 at 163,842, 77 and 70 at 655,362.
+static bool two_waves(const gs_plan* p, int blocks) { return p->n > (int64_t)2 * p->sm_count * blocks * 128; }
+
 // `post` runs in the receivers' kernel where *fused comes back true
 static int receivers_post(gs_plan* p, int nrcv, double exp, const double* elev, double sl, const int* gid, int* rcv,
                           double* dist, double* wgt, int8_t* rslot, const DirPost& post, bool* fused) {
@@ -502,19 +538,24 @@ static int receivers_post(gs_plan* p, int nrcv, double exp, const double* elev, 
         else if (p->W <= 8) f(std::integral_constant<int, 8>{});
         else f(std::integral_constant<int, 12>{});
     };
+    auto ranked = [&](auto w) {
+        constexpr int NP = decltype(w)::value;
+        launch(p, nrcv == 1 ? k_mfd_receivers_r<1, NP> : nrcv == 2 ? k_mfd_receivers_r<2, NP>
+                  : nrcv == 3 ? k_mfd_receivers_r<3, NP> : k_mfd_receivers_r<4, NP>,
+               G, 128, n, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt, rslot, post);
+    };
     if (nrcv >= p->W)
         width([&](auto w) {
-            launch(p, k_mfd_all<decltype(w)::value>, G, 128, n, nrcv, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv,
-                   dist, wgt, rslot, post);
-        });
-    else if (nrcv <= 4)
-        width([&](auto w) {
             constexpr int NP = decltype(w)::value;
-            launch(p, nrcv == 1 ? k_mfd_receivers_r<1, NP> : nrcv == 2 ? k_mfd_receivers_r<2, NP>
-                      : nrcv == 3 ? k_mfd_receivers_r<3, NP> : k_mfd_receivers_r<4, NP>,
-                   G, 128, n, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt, rslot, post);
+            constexpr int FEW = NP == 6 ? 8 : 1, MANY = NP == 12 ? 6 : 8;
+            launch(p, two_waves(p, 4) ? k_mfd_all<NP, MANY> : k_mfd_all<NP, FEW>, G, 128, n, nrcv, exp, elev, sl, g,
+                   p->nbr, p->elen, p->nnb, rcv, dist, wgt, rslot, post);
         });
-    else
+    else if (nrcv <= 4) {
+        const bool loop = p->W <= 6 ? nrcv == 4 && two_waves(p, 8) : two_waves(p, p->W <= 8 && nrcv <= 3 ? 5 : 4);
+        if (loop) ranked(std::integral_constant<int, 0>{});
+        else width(ranked);
+    } else
         launch(p, k_mfd_receivers, G, 128, n, p->W, nrcv, exp, elev, sl, g, p->nbr, p->elen, p->nnb, rcv, dist, wgt,
                rslot);
     GS_LAUNCH();
