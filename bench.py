@@ -990,11 +990,15 @@ def _short(name):
     for tok in s.replace("(", " ").replace("<", " ").split():
         if tok.startswith("_ZN2gs"):
             rest = tok[6:]
-            ln = ""
-            while rest and rest[0].isdigit():
-                ln += rest[0]
-                rest = rest[1:]
-            return rest[:int(ln)] if ln else tok
+            while True:
+                ln = ""
+                while rest and rest[0].isdigit():
+                    ln += rest[0]
+                    rest = rest[1:]
+                part = rest[:int(ln)] if ln else tok
+                if not part.startswith("_GLOBAL__N_"):   # the kernels of gs_tiles.cu
+                    return part
+                rest = rest[int(ln):]
         if tok.startswith("gs::"):
             return tok[4:]
     return s

@@ -1,10 +1,11 @@
 """Launch-shape autotuner.
 
-The ordered dependency sweeps and the cooperative kernels (basin relaxation,
-grid BFS, hillslope CG) have a free launch shape: blocks per SM.  More blocks
-keep more dependency chains in flight but compete for the SM with the kernels
-running beside them on the side streams; the best shape depends on the mesh
-(DAG depth, pit structure) and the GPU.  ``tune(model)`` times a few physics
+The ordered dependency sweeps (meshes too large for tiles, the FP32 form) and the
+cooperative diffusion solves have a free launch shape: blocks, or groups of 256
+threads, per SM.  More of them keep more dependency chains in flight but compete
+for the SM with the kernels running beside them on the side streams; the best
+shape depends on the mesh (DAG depth, pit structure) and the GPU.  Where the sweeps
+run on mesh tiles only the second knob matters.  ``tune(model)`` times a few physics
 steps for each candidate on the model's own landscape, restores the state
 after every trial, and keeps the fastest shape in the plan.  The knobs change
 launch shapes only; results change only by the rounding of the hillslope CG's

@@ -960,14 +960,8 @@ int hillslope(gs_plan* p, double* h, double* cum_ed, double* eb, double sealevel
     return GS_OK;
 }
 
-// Solve (I + L) x = rhs on a sub-mesh of m rows given as rows (diag, then
-// one coefficient per neighbour slot, [W+1][m], the hillslope layout; slot-major
-// [W][m] neighbours, -1 or a zero coefficient where a neighbour lies outside),
-// rows without area held fixed as in the hillslope solve; the cooperative CG on
-// the area-weighted symmetric form.  Used by the non-linear lake diffusion of
-// the sediment step.
-// the lagged-diffusivity solves over the m cells `cell` (k_picard), the worst
-// relative residual (NaN wins) in *worst on the device
+// The lagged-diffusivity solves of the lake and marine deposits over the m cells
+// `cell` (k_picard); the worst relative residual (NaN wins) in *worst on the device.
 int picard_solve(gs_plan* p, int m, const int* cell, const int* nbr, const int8_t* nnb, const double* farea,
                  const uint8_t* fix, const double* zb, double K, double dts, double* hcur, double* cd, double* hs,
                  double* coef, double rtol, int max_iter, double* worst) {
@@ -980,6 +974,11 @@ int picard_solve(gs_plan* p, int m, const int* cell, const int* nbr, const int8_
     return cg_launch(p, (const void*)k_picard, ng, args);
 }
 
+// Solve (I + L) x = rhs on a sub-mesh of m rows given as rows (diag, then
+// one coefficient per neighbour slot, [W+1][m], the hillslope layout; slot-major
+// [W][m] neighbours, -1 or a zero coefficient where a neighbour lies outside),
+// rows without area held fixed as in the hillslope solve; the cooperative CG on
+// the area-weighted symmetric form.  Used by the smoothing of the marine surface.
 int diffusion_solve_on(gs_plan* p, int m, const int* nbr, const int8_t* nnb, const double* farea, const uint8_t* fix,
                        int flat, const uint8_t* outlet, const double* coef, const double* rhs, double* x, double rtol,
                        int max_iter, int* iters, const double* guess) {

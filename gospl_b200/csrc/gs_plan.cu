@@ -448,7 +448,7 @@ int plan_tune(gs_plan* p, int knob, int value) {
     }
     if (knob == GS_TUNE_FLAT_BFS) {
         if (value < 0 || value > 4096) {
-            set_error(GS_EINVAL, "tune: flat BFS must be 0 (one block) or a window of 1..4096 levels (tiles)");
+            set_error(GS_EINVAL, "tune: flat search must be 0 (by depression) or a window of 1..4096 levels (tiles)");
             return GS_EINVAL;
         }
         p->bfs_window = value;

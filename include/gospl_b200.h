@@ -40,7 +40,7 @@ typedef struct gs_stats {
     int32_t npits;            /* depressions found by the fill (P; ids 1..P)          */
     int32_t cascade_passes;   /* _distributeDownstream passes executed                */
     int32_t cascade_solves;   /* cascade flow solves executed                         */
-    int32_t fill_rounds;      /* spill-graph relaxation rounds                        */
+    int32_t fill_rounds;      /* rounds over the basin graph                          */
     int32_t flat_rounds;      /* flat-distance BFS levels                             */
     int32_t cycle_nodes;      /* nodes solved by the cycle fallback (0 when acyclic)  */
     int32_t cg_iters;         /* hillslope CG iterations                              */
@@ -81,9 +81,10 @@ int gs_plan_set_stream(gs_plan* plan, void* cuda_stream);
 /*
  * Launch-shape knobs (no counterpart in the reference).  GS_TUNE_SWEEP_BLOCKS:
  * 128-thread blocks per SM of the ordered dependency sweeps (1..32, default
- * 8).  GS_TUNE_COOP_BLOCKS: 256-thread blocks per SM of the cooperative
- * kernels (basin relaxation, grid BFS, hillslope CG; 1..their co-residency
- * limit, default min(limit, 4)); gs_plan_tuning(plan, GS_TUNE_COOP_BLOCKS + 1)
+ * 8); without effect where the sweeps run on mesh tiles.
+ * GS_TUNE_COOP_BLOCKS: groups of 256 threads per SM of the diffusion solves, and
+ * blocks of the basin relaxation of meshes with one-sided edges (1..their
+ * co-residency limit, default min(limit, 4)); gs_plan_tuning(plan, GS_TUNE_COOP_BLOCKS + 1)
  * returns that limit.  Results do not depend on the knobs beyond the
  * rounding of the hillslope CG's inner products (block partial sums); speed
  * does (gospl_b200.autotune picks them by timing steps).
@@ -96,7 +97,8 @@ int gs_plan_set_stream(gs_plan* plan, void* cuda_stream);
                                      still waiting on a predecessor after it stops with GS_ETIMEOUT */
 #define GS_TUNE_FLAT_BFS 7        /* flat-distance search: 0 by depression (default), w in 1..4096 over all
                                      depressions in tiles, one cooperative launch settling distance windows
-                                     of w levels */
+                                     of w levels.  At 0 a mesh with one-sided edges, or a lake of more than
+                                     1,048,576 cells, is searched over all depressions too */
 #define GS_TUNE_WARM_START 8      /* 1 (default): the hillslope CG starts from h plus the previous step's
                                      diffusion change and the bathymetry smoothing from the previous
                                      smoothing; 0: both start from their right-hand side, so that a step
