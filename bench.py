@@ -1070,10 +1070,9 @@ def step_algo_bytes(L):
 # launch divided by the vertices it processed) from the ncu captures summarised
 # under profiles/; scaled by the vertex count of the run.
 NCU_TRAFFIC_PER_VERTEX = {
-    "k_mfd_receivers": (24.905728e6 + 2.152192e6) / 655362,
+    "k_mfd_receivers": (40.322304e6 + 4.224256e6) / 655362,
     "k_ordered_flow": (38.153216e6 + 1.851392e6) / 655362,
     "k_bfs_local": 1.780992e6 / 655362,
-    "k_relax_active": (1.359360e6 + 0.125440e6) / 655362,
 }
 
 
